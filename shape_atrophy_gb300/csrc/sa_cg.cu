@@ -40,13 +40,6 @@
 
 namespace sa {
 
-struct CgScal {
-	double bb, rr, gam, gamPrev, alpha, beta, delta, tolSqu;
-	int first, done, code, iters, zero, itrMax;
-	unsigned int counter;
-	int pad;
-};
-
 // FP64 throughput on GB300 is 2 thread-DFMA per clock per SM (a warp
 // instruction occupies the SM's FP64 pipe for 16 cycles), so the kernels
 // below avoid FP64 work that is not the algorithm's own: in the two-kernel
@@ -1364,6 +1357,33 @@ static CgScal run_cg(const Mesh &m, const TM *blk, const TV *dinv, const double 
 		binv = sizeof(TV) == sizeof(float) ? (const TV *) (const void *) prof->binv32
 		                                   : (const TV *) (const void *) prof->binv64;
 		if (!binv) throw CudaError{cudaErrorInvalidValue, "block-Jacobi CG without block inverses"};
+	}
+	// FP64 velocity solves: the persistent CG with fixed-point matrix products, where its plan exists (at most one
+	// slice per row warp and a halo that fits shared memory)
+	if constexpr (B > 1 && sizeof(TM) == sizeof(double) && sizeof(TX) == sizeof(double)) {
+		if (prof->plan.ok && prof->bar && (prof->cgKernel == SA_CG_AUTO || prof->cgKernel == SA_CG_PERSISTENT)) {
+			k_cg_init_blk<B, TV><<<vec_grid(N, prof->smCount), kCgBlock, 0, s>>>(N, b, q, binv, r, u, part, sc);
+			if (cgfix_run<B>(m, blk, binv, x, r, u, *prof, timing ? prof->ev[0] : nullptr, timing ? prof->ev[1] : nullptr, s)) {
+				k_cg_zero<TX><<<grid_for(n), kBlock, 0, s>>>(n, x, sc);
+				prof->launches += 2;
+				unsigned int gaveUp = 0;
+				SA_CHECK(cudaMemcpyAsync(&gaveUp, &((GridBar *) prof->bar)->abort, sizeof(unsigned int),
+				                         cudaMemcpyDeviceToHost, s));
+				CgScal h = read_scal(sc, s);
+				if (timing && h.iters > 0) {
+					float ms = 0.f;
+					SA_CHECK(cudaEventElapsedTime(&ms, prof->ev[0], prof->ev[1]));
+					prof->spmvMs += ms;
+					prof->spmvCount += 1;
+					// per iteration: operator digits once, u gathered once and written once; per launch: x, r, u in, x out
+					prof->profBytes += (double) h.iters * ((double) prof->plan.total * B * B * sizeof(TM) + 2.0 * sizeof(TV) * n) +
+					                   4.0 * sizeof(TV) * n;
+					prof->profFlops += (double) h.iters * 2.0 * ((double) B * B * m.slTotal + (7.0 + B) * n);
+				}
+				if (gaveUp || h.code == SA_ERR_TIMEOUT) throw DeviceWaitError{"persistent CG grid barrier"};
+				return h;
+			}
+		}
 	}
 	// persistent launch: one CTA per SM, one slice per row warp plus the reducer warp
 	const int pwCap = std::max(1, std::min(kPersistMaxWarps, tuning().persistMaxWarps) - 1);

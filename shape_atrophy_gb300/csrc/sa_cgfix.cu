@@ -1,0 +1,790 @@
+// sa_cgfix.cu -- persistent block-Jacobi CG whose matrix products are summed in fixed point.
+//
+// The FP64 velocity solve of k_cg_persist (sa_cg.cu) is bound by the FP64 pipe: 9 multiply-adds per 3 x 3 block
+// at 64 clocks per warp and SM sub-partition, 22 of the 35 us of an iteration on the 92 178-node shell, against
+// 6 us for reading the operator (94 MB) from the L2.  Here the products go through the integer pipes
+// (sa_limb.cuh), which takes them off the critical path and leaves the loads:
+//   * the operator is converted once per solve to two 28-bit digits per entry (k_cgfix_operator; the bytes of
+//     the FP64 entry).  A slice that fits its warp's ring of slots in shared memory stays there for the whole solve;
+//     of larger ones as many slots as fit stay in tensor memory (39 MB over the chip: with the operator, the vectors
+//     and u the working set of the shell is 107 MB, beyond what the L2 holds of a cyclic scan), and the rest is
+//     streamed by bulk copies into the ring, ahead of its use and across the grid barriers;
+//   * the vector u is converted once per CTA and iteration: the distinct nodes a chunk's rows gather (its
+//     halo, about 1.7 times its rows in Morton order; in the icosphere's own numbering nearly every slot is a node of
+//     its own) are read into shared memory as two 28-bit digits relative to the halo's largest entry, so a
+//     slot's gather is six shared-memory words instead of two L2 requests;
+//   * the two grid sums of an iteration carry their own barrier (sum_exchange in sa_grid.cuh).
+// The recurrences, the reducer warp and the stopping rule are those of k_cg_persist (sa_cg.cu): Chronopoulos-Gear
+// in FP64, exact grid sums, bounded waits.
+#include "sa_internal.cuh"
+#include "sa_grid.cuh"
+#include "sa_limb.cuh"
+#include <algorithm>
+#include <mutex>
+
+namespace sa {
+
+constexpr int kFixMaxWarps = 20;           // CTA size limit, reducer warp included (as the persistent CG's)
+constexpr int kFixMinWarps = 8;            // small solves: warps without rows help to stage the halo
+constexpr int kFixMaxParts = 8;            // warps per slice
+constexpr int kFixMaxHalo = 8192;          // halo nodes per chunk (shared memory takes about 6000 of them)
+constexpr int kFixMaxRows = 1 << 20;       // permuted rows whose bit map and prefix counts fit shared memory
+
+template <int B> constexpr int limb_stride() { return 6; }    // words per halo node: three 8-byte bank pairs, odd, so consecutive nodes spread
+template <int B> constexpr int fix_u_stride() { return B == 3 ? 4 : 2; }   // doubles per node of the gather copy
+
+// ---------------------------------------------------------------------------
+// plan
+// ---------------------------------------------------------------------------
+// one CTA per chunk: its rows sorted by length (longest first, ties in Morton order)
+__global__ void k_plan_rows(int N, int nchunk, int R, const unsigned long long *__restrict__ keys,
+                            const int *__restrict__ rowPtr, int *__restrict__ perm, int *__restrict__ inv,
+                            int *__restrict__ width)
+{
+	extern __shared__ int sh[];
+	int *deg = sh, *sorted = sh + R;
+	const int c = blockIdx.x, r0 = (int) ((long) c * N / nchunk), n = (int) ((long) (c + 1) * N / nchunk) - r0;
+	for (int t = threadIdx.x; t < n; t += blockDim.x) {
+		const int i = (int) (keys[r0 + t] & 0xffffffffu);
+		deg[t] = rowPtr[i + 1] - rowPtr[i];
+	}
+	__syncthreads();
+	for (int t = threadIdx.x; t < R; t += blockDim.x) {
+		if (t >= n) { perm[(long) c * R + t] = -1; continue; }
+		const int d = deg[t], i = (int) (keys[r0 + t] & 0xffffffffu);
+		int rank = 0;
+		for (int q = 0; q < n; ++q) rank += deg[q] > d || (deg[q] == d && q < t);
+		perm[(long) c * R + rank] = i;
+		inv[i] = c * R + rank;
+		sorted[rank] = d;
+	}
+	__syncthreads();
+	for (int q = threadIdx.x; q < R / 32; q += blockDim.x) width[c * (R / 32) + q] = 32 * q < n ? sorted[32 * q] : 0;
+}
+
+// first slot of every slice (one CTA); off[ns] = total
+__global__ void __launch_bounds__(1024) k_plan_offsets(int ns, const int *__restrict__ width, int *__restrict__ off)
+{
+	__shared__ int sum[1024];
+	const int t = threadIdx.x, per = (ns + 1023) / 1024, a = min(ns, t * per), b = min(ns, a + per);
+	int s = 0;
+	for (int q = a; q < b; ++q) s += 32 * width[q];
+	sum[t] = s;
+	__syncthreads();
+	for (int h = 1; h < 1024; h <<= 1) {
+		const int v = t >= h ? sum[t - h] : 0;
+		__syncthreads();
+		sum[t] += v;
+		__syncthreads();
+	}
+	int o = sum[t] - s;
+	for (int q = a; q < b; ++q) { off[q] = o; o += 32 * width[q]; }
+	if (t == 1023) off[ns] = sum[1023];
+}
+
+// one CTA per chunk: the distinct columns of its rows (bit map over the permuted rows, prefix counts per word),
+// its halo list, and every slot's place in that list (padding slots: place 0, their entries are zero)
+__global__ void k_plan_columns(int P, int R, const int *__restrict__ rowPtr, const int *__restrict__ col,
+                               const int *__restrict__ perm, const int *__restrict__ inv,
+                               const int *__restrict__ width, const int *__restrict__ off, int haloCap,
+                               int *__restrict__ halo, int *__restrict__ haloNum, unsigned short *__restrict__ lcol)
+{
+	extern __shared__ int sh[];
+	__shared__ int part[1025];
+	const int nw = (P + 31) / 32, c = blockIdx.x, t0 = threadIdx.x, nt = blockDim.x;
+	unsigned *bits = (unsigned *) sh;
+	unsigned short *pre = (unsigned short *) (sh + nw);
+	for (int w = t0; w < nw; w += nt) bits[w] = 0u;
+	__syncthreads();
+	for (int t = t0; t < R; t += nt) {
+		const int i = perm[(long) c * R + t];
+		if (i < 0) continue;
+		for (int z = rowPtr[i]; z < rowPtr[i + 1]; ++z) {
+			const int q = inv[col[z]];
+			atomicOr(&bits[q >> 5], 1u << (q & 31));
+		}
+	}
+	__syncthreads();
+	const int per = (nw + nt - 1) / nt, a = min(nw, t0 * per), b = min(nw, a + per);
+	int s = 0;
+	for (int w = a; w < b; ++w) s += __popc(bits[w]);
+	part[t0 + 1] = s;
+	if (t0 == 0) part[0] = 0;
+	__syncthreads();
+	if (t0 == 0)
+		for (int k = 1; k <= nt; ++k) part[k] += part[k - 1];
+	__syncthreads();
+	int o = part[t0];
+	for (int w = a; w < b; ++w) {
+		pre[w] = (unsigned short) min(o, 65535);
+		for (unsigned m = bits[w]; m; m &= m - 1u) {
+			if (o < haloCap) halo[(long) c * haloCap + o] = 32 * w + __ffs((int) m) - 1;
+			++o;
+		}
+	}
+	if (t0 == 0) haloNum[c] = part[nt];
+	__syncthreads();
+	for (int t = t0; t < R; t += nt) {
+		const int i = perm[(long) c * R + t], sl = c * (R / 32) + t / 32, w = width[sl];
+		const long base = off[sl] + (t & 31);
+		const int z0 = i >= 0 ? rowPtr[i] : 0, len = i >= 0 ? rowPtr[i + 1] - z0 : 0;
+		for (int k = 0; k < w; ++k) {
+			int h = 0;
+			if (k < len) {
+				const int q = inv[col[z0 + k]];
+				h = pre[q >> 5] + __popc(bits[q >> 5] & ((1u << (q & 31)) - 1u));
+			}
+			lcol[base + 32L * k] = (unsigned short) h;
+		}
+	}
+}
+
+static size_t fix_smem_limit(const void *kernel)
+{
+	int dev = 0, optin = 0;
+	cudaFuncAttributes fa;
+	if (cudaGetDevice(&dev) != cudaSuccess ||
+	    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+	    cudaFuncGetAttributes(&fa, kernel) != cudaSuccess || (size_t) optin <= fa.sharedSizeBytes) {
+		cudaGetLastError();
+		return 0;
+	}
+	const size_t want = (size_t) optin - fa.sharedSizeBytes;
+	if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) want) != cudaSuccess) {
+		cudaGetLastError();
+		return 0;
+	}
+	return want;
+}
+
+bool cgfix_plan(const Mesh &m, const double *x0soa, int smCount, int maxWarps, CgPlan &p,
+                const std::function<void *(size_t)> &alloc, cudaStream_t s)
+{
+	p = CgPlan();
+	const int B = m.dim, ns0 = (m.N + 31) / 32;
+	const int cap = std::min(kFixMaxWarps, maxWarps) - 1;
+	if (cap < 1 || smCount < 1) return false;
+	p.pw = std::max(1, (ns0 + smCount - 1) / smCount);
+	if (p.pw > cap) return false;
+	p.nchunk = (ns0 + p.pw - 1) / p.pw;
+	for (size_t q = 0; q + 1 < m.slOffHost.size(); ++q)
+		p.widest = std::max(p.widest, (m.slOffHost[q + 1] - m.slOffHost[q]) / 32);
+	// small chunks: several warps share a slice, two slots or more each (a slot costs one warp about 450 clocks of
+	// latency, against 160 of issue; the digit sums are integers, so the split changes no bit)
+	p.parts = std::max(1, std::min({cap / p.pw, kFixMaxParts, (p.widest + 1) / 2}));
+	p.warps = std::max(std::min(kFixMinWarps, maxWarps), p.pw * p.parts + 1);
+	p.nslice = p.nchunk * p.pw;
+	p.haloCap = std::min(kFixMaxHalo, p.nchunk * 32 * p.pw);
+	const int R = 32 * p.pw, P = p.nchunk * R;
+	if (P > kFixMaxRows || p.widest * B > kLimbMaxTerms) return false;
+	auto get = [&](size_t bytes) { return alloc(std::max<size_t>(bytes, 16)); };
+	double *scr = (double *) get(sizeof(double) * morton_order_doubles(B, m.N));
+	p.perm = (int *) get(sizeof(int) * (size_t) P);
+	p.inv = (int *) get(sizeof(int) * (size_t) m.N);
+	p.width = (int *) get(sizeof(int) * (size_t) p.nslice);
+	p.off = (int *) get(sizeof(int) * (size_t) (p.nslice + 1));
+	p.halo = (int *) get(sizeof(int) * (size_t) p.nchunk * p.haloCap);
+	p.haloNum = (int *) get(sizeof(int) * (size_t) p.nchunk);
+	if (!scr || !p.perm || !p.inv || !p.width || !p.off || !p.halo || !p.haloNum) return false;
+	const unsigned long long *keys = B == 2 ? morton_order<2>(m.N, x0soa, scr, s) : morton_order<3>(m.N, x0soa, scr, s);
+	k_plan_rows<<<p.nchunk, 256, 2 * sizeof(int) * R, s>>>(m.N, p.nchunk, R, keys, m.rowPtr, p.perm, p.inv, p.width);
+	k_plan_offsets<<<1, 1024, 0, s>>>(p.nslice, p.width, p.off);
+	int total = 0;
+	SA_CHECK(cudaMemcpyAsync(&total, p.off + p.nslice, sizeof(int), cudaMemcpyDeviceToHost, s));
+	SA_CHECK(cudaStreamSynchronize(s));
+	p.total = total;
+	p.lcol = (unsigned short *) get(sizeof(unsigned short) * (size_t) total);
+	p.fix = (int2 *) get(sizeof(int2) * (size_t) total * B * B);
+	p.rowExp = (int *) get(sizeof(int) * (size_t) P);
+	p.ug = (double *) get(sizeof(double) * (size_t) P * (B == 3 ? fix_u_stride<3>() : fix_u_stride<2>()));
+	p.vec = (double *) get(sizeof(double) * (size_t) P * 4 * B);
+	if (!p.lcol || !p.fix || !p.rowExp || !p.ug || !p.vec) return false;
+	const int nw = (P + 31) / 32;
+	const size_t sm = sizeof(int) * (size_t) nw + sizeof(unsigned short) * (size_t) (nw + 1);
+	if (sm > 48 * 1024 && sm > fix_smem_limit((const void *) k_plan_columns)) return false;
+	k_plan_columns<<<p.nchunk, 512, sm, s>>>(P, R, m.rowPtr, m.femVtx + m.Z, p.perm, p.inv, p.width, p.off, p.haloCap,
+	                                         p.halo, p.haloNum, p.lcol);
+	SA_CHECK(cudaGetLastError());
+	std::vector<int> num(p.nchunk);
+	SA_CHECK(cudaMemcpyAsync(num.data(), p.haloNum, sizeof(int) * p.nchunk, cudaMemcpyDeviceToHost, s));
+	SA_CHECK(cudaStreamSynchronize(s));
+	for (int c : num) p.haloMax = std::max(p.haloMax, c);
+	p.ok = p.haloMax <= p.haloCap;
+	return p.ok;
+}
+
+// ---------------------------------------------------------------------------
+// operator: the permuted rows' entries as digits, and the row frames.  One warp per slice.
+// ---------------------------------------------------------------------------
+template <int B>
+__global__ void __launch_bounds__(128) k_cgfix_operator(int nslice, SellOp A, const int *__restrict__ rowPtr,
+                                                        const double *__restrict__ blk, const int *__restrict__ perm,
+                                                        const int *__restrict__ width, const int *__restrict__ off,
+                                                        int2 *__restrict__ fix, int *__restrict__ rowExp)
+{
+	const int sl = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+	if (sl >= nslice) return;
+	const int i = perm[(long) sl * 32 + lane], w = width[sl];
+	const int len = i >= 0 ? rowPtr[i + 1] - rowPtr[i] : 0;
+	const double *row = blk + (i >= 0 ? ((long) __ldg(A.off + (i >> 5))) * (B * B) + (i & 31) : 0l);
+	int e = 1;
+	for (int k = 0; k < len; ++k)
+		for (int t = 0; t < B * B; ++t) e = max(e, fx_exp(__ldg(row + ((long) k * B * B + t) * 32)));
+	rowExp[(long) sl * 32 + lane] = e;
+	int2 *o = fix + (long) off[sl] * (B * B) + lane;
+	for (int k = 0; k < w; ++k)
+		for (int t = 0; t < B * B; ++t) {
+			int2 d = make_int2(0, 0);
+			if (k < len && e < 2047) limb_matrix(__ldg(row + ((long) k * B * B + t) * 32), e, d.x, d.y);
+			o[((long) k * B * B + t) * 32] = d;
+		}
+}
+
+// u (natural order, stride B) -> its gather copy in permuted order
+template <int B>
+__global__ void k_cgfix_gather_copy(int P, const int *__restrict__ perm, const double *__restrict__ u,
+                                    double *__restrict__ ug)
+{
+	const int q = blockIdx.x * blockDim.x + threadIdx.x;
+	if (q >= P) return;
+	const int i = perm[q];
+	for (int c = 0; c < fix_u_stride<B>(); ++c)
+		ug[(long) q * fix_u_stride<B>() + c] = i >= 0 && c < B ? u[(long) i * B + c] : 0.0;
+}
+
+// ---------------------------------------------------------------------------
+// the solve
+// ---------------------------------------------------------------------------
+struct FixArgs {
+	int pw, parts, haloCap, haloMax, colMax, stages;
+	const int *perm, *width, *off, *halo, *haloNum, *rowExp;
+	const unsigned short *lcol;
+	const int2 *fix;
+	const double *binv, *r0, *u0;
+	double *x, *ug, *vec, *part;
+	CgScal *sc;
+	GridSums *gs;
+};
+
+// shared memory of one CTA in bytes: operator ring, block inverses, u, ring barriers, the
+// other parts' digit sums, halo digits and rows, slot places
+template <int B> size_t fix_smem(int pw, int parts, int haloMax, int colMax, int stages)
+{
+	return (size_t) pw * stages * (256 * B * B + 8) + sizeof(double) * (size_t) pw * 32 * (B * B + B + (parts - 1) * 3 * B) +
+	       sizeof(int) * (size_t) haloMax * (limb_stride<B>() + 1) + sizeof(unsigned short) * (size_t) colMax + 16;
+}
+
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned) __cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void ring_load(void *dst, const void *src, unsigned bytes, unsigned bar)
+{
+	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
+	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+	             :: "r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+constexpr int kRingTries = 1 << 20;        // bounded wait: each try suspends up to a hardware time limit
+__device__ __forceinline__ bool ring_wait(unsigned bar, unsigned parity)
+{
+	for (int n = 0; n < kRingTries; ++n) {
+		unsigned ok;
+		asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+		             : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+		if (ok) return true;
+	}
+	return false;
+}
+
+// acc += block a (shared memory, [entry][lane]) times the node's digits u
+template <int B>
+__device__ __forceinline__ void fix_slot_mac(LimbSum (&acc)[B], const int2 *__restrict__ a, const int *__restrict__ u)
+{
+#pragma unroll
+	for (int c = 0; c < B; ++c) {
+		const int2 ud = reinterpret_cast<const int2 *>(u)[c];
+		const int u1 = ud.x, u0 = ud.y;
+#pragma unroll
+		for (int r = 0; r < B; ++r) {
+			const int2 e = a[(r * B + c) * 32];
+			limb_mac(acc[r], e.x, e.y, u1, u0);
+		}
+	}
+}
+
+// Operator slots kept in tensor memory (256 KB per SM, otherwise idle here): warp w of the CTA reaches the 32 lanes
+// of its quarter w % 4, one lane per row, 2 B B columns per slot (digits of the block's entries, column by column).
+constexpr int kTmemCols = 512;
+
+// slots of one warp in tensor memory: the quarter's columns are shared by (pw + 3) / 4 row warps
+template <int B> __host__ __device__ constexpr int tmem_slots(int pw) { return kTmemCols / (2 * B * B * ((pw + 3) / 4)); }
+
+template <int B> __device__ __forceinline__ void tmem_store(unsigned t, const int2 (&e)[B * B])
+{
+	if constexpr (B == 3)
+		asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n"
+		             "tcgen05.st.sync.aligned.32x32b.x2.b32 [%17], {%18, %19};\n"
+		             "tcgen05.wait::st.sync.aligned;"
+		             :: "r"(t), "r"(e[0].x), "r"(e[0].y), "r"(e[1].x), "r"(e[1].y), "r"(e[2].x), "r"(e[2].y), "r"(e[3].x), "r"(e[3].y),
+		                "r"(e[4].x), "r"(e[4].y), "r"(e[5].x), "r"(e[5].y), "r"(e[6].x), "r"(e[6].y), "r"(e[7].x), "r"(e[7].y),
+		                "r"(t + 16), "r"(e[8].x), "r"(e[8].y) : "memory");
+	else
+		asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
+		             "tcgen05.wait::st.sync.aligned;"
+		             :: "r"(t), "r"(e[0].x), "r"(e[0].y), "r"(e[1].x), "r"(e[1].y), "r"(e[2].x), "r"(e[2].y), "r"(e[3].x), "r"(e[3].y)
+		             : "memory");
+}
+
+template <int B> __device__ __forceinline__ void tmem_load(unsigned t, int2 (&e)[B * B])
+{
+	if constexpr (B == 3)
+		asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%18];\n"
+		             "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%16, %17}, [%19];\n"
+		             "tcgen05.wait::ld.sync.aligned;"
+		             : "=r"(e[0].x), "=r"(e[0].y), "=r"(e[1].x), "=r"(e[1].y), "=r"(e[2].x), "=r"(e[2].y), "=r"(e[3].x), "=r"(e[3].y),
+		               "=r"(e[4].x), "=r"(e[4].y), "=r"(e[5].x), "=r"(e[5].y), "=r"(e[6].x), "=r"(e[6].y), "=r"(e[7].x), "=r"(e[7].y),
+		               "=r"(e[8].x), "=r"(e[8].y) : "r"(t), "r"(t + 16));
+	else
+		asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+		             "tcgen05.wait::ld.sync.aligned;"
+		             : "=r"(e[0].x), "=r"(e[0].y), "=r"(e[1].x), "=r"(e[1].y), "=r"(e[2].x), "=r"(e[2].y), "=r"(e[3].x), "=r"(e[3].y)
+		             : "r"(t));
+}
+
+// acc += the block in e (tensor memory order: column by column) times the node's digits u
+template <int B>
+__device__ __forceinline__ void tmem_slot_mac(LimbSum (&acc)[B], const int2 (&e)[B * B], const int *__restrict__ u)
+{
+#pragma unroll
+	for (int c = 0; c < B; ++c) {
+		const int2 ud = reinterpret_cast<const int2 *>(u)[c];
+		const int u1 = ud.x, u0 = ud.y;
+#pragma unroll
+		for (int r = 0; r < B; ++r) limb_mac(acc[r], e[c * B + r].x, e[c * B + r].y, u1, u0);
+	}
+}
+
+// a halo node's u, written by other CTAs during the launch: one request, through L2
+template <int B> __device__ __forceinline__ void load_halo(const double *p, double (&v)[B])
+{
+	if constexpr (B == 3) {
+		double pad;
+		asm volatile("ld.relaxed.gpu.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+		             : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(pad) : "l"(p) : "memory");
+	} else {
+		const double2 t = __ldcg(reinterpret_cast<const double2 *>(p));
+		v[0] = t.x;
+		v[1] = t.y;
+	}
+}
+
+// the partial-sum path of a grid sum (no frame yet, or a value out of its frame); called by every thread of every CTA
+template <int K>
+__device__ __noinline__ bool slow_sum(double a, double b, double *res, double *part, int nctas, GridBar *bar,
+                                      unsigned &target, FxScratch &fs)
+{
+	double v[K], t[K];
+	v[0] = a;
+	if (K > 1) v[K - 1] = b;
+	if (!grid_reduce<K, double>(v, t, part, blockIdx.x, nctas, bar, target, fs)) return false;
+	if (threadIdx.x == 0)
+		for (int k = 0; k < K; ++k) res[k] = t[k];
+	__syncthreads();
+	return true;
+}
+
+// kStream: the ring does not hold every slot of a slice
+template <int B, bool kStream>
+__global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a)
+{
+	__shared__ FxScratch fs;
+	__shared__ unsigned dig[kFixMaxWarps][kSumWords];
+	// the iteration's scalars, written by the reducer warp
+	__shared__ double gam, rr, beta, dsub, alpha, delta, two[2];   // dsub = beta * gamma / alphaPrev
+	__shared__ double goal;                      // squared residual to reach
+	__shared__ int itrMax, stop, broke, iters, gaveUp, slow, sE[32];
+	__shared__ unsigned tmemBase;
+	extern __shared__ __align__(128) char sdyn[];
+	CgScal *sc = a.sc;
+	if (sc->done) return;                        // set by k_cg_init: the same for every CTA
+	constexpr int S = limb_stride<B>(), U = fix_u_stride<B>(), BB = B * B;
+	constexpr unsigned kSlot = 256 * BB;         // bytes of one slot of a slice
+	const int nctas = gridDim.x, lc = blockIdx.x, pw = a.pw;
+	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, W = blockDim.x >> 5;
+	// warps 0 .. pw - 1 own one slice each; the next pw (parts - 1) warps share their slots; then warps that only stage
+	const bool reducer = wp == W - 1, rowWarp = wp < pw, worker = wp < pw * a.parts;
+	const int ws = kStream ? wp : wp % pw, part = kStream ? 0 : wp / pw;
+	// shared memory: offsets from sdyn
+	const int oInv = pw * a.stages * (int) kSlot, oU = oInv + pw * 256 * BB, oBar = oU + pw * 256 * B;
+	const int oPart = oBar + 8 * pw * a.stages, oLimb = oPart + (a.parts - 1) * pw * 768 * B, oHalo = oLimb + 4 * a.haloMax * S, oCol = oHalo + 4 * a.haloMax;
+	int *slimb = (int *) (sdyn + oLimb), *shalo = (int *) (sdyn + oHalo);
+	unsigned short *scol = (unsigned short *) (sdyn + oCol);
+	double *su = (double *) (sdyn + oU) + wp * B * 32 + lane;            // row warps only
+	char *ring = sdyn + ws * a.stages * (int) kSlot;
+	const unsigned mb = smem_addr(sdyn + oBar + 8 * ws * a.stages);
+	const int sl = lc * pw + ws, row = sl * 32 + lane;        // permuted row (workers)
+	const int i = rowWarp ? __ldg(a.perm + row) : -1;
+	const bool own = i >= 0;
+	const int wdt = worker ? __ldg(a.width + sl) : 0;
+	const int o0 = __ldg(a.off + lc * pw);
+	const int o1 = worker ? __ldg(a.off + sl) : o0;
+	const char *src = (const char *) a.fix + (size_t) o1 * (8 * BB);
+	const unsigned short *mycol = scol + (o1 - o0) + lane;
+	const int eRow = rowWarp ? __ldg(a.rowExp + row) : 1;
+	const int nhalo = __ldg(a.haloNum + lc);
+	for (int t = threadIdx.x, n = __ldg(a.off + (lc + 1) * pw) - o0; t < n; t += blockDim.x) scol[t] = __ldg(a.lcol + o0 + t);
+	for (int t = threadIdx.x; t < nhalo; t += blockDim.x) shalo[t] = __ldg(a.halo + (long) lc * a.haloCap + t);
+	if (threadIdx.x == 0) {
+		gam = sc->gam; rr = sc->rr; beta = 0.0; dsub = 0.0; alpha = 1.0; delta = 0.0;
+		goal = sc->tolSqu * sc->bb; itrMax = sc->itrMax;
+		stop = -1; broke = -1; iters = 0; gaveUp = 0; slow = 0;
+	}
+	// operator: the warp's last ntm slots in tensor memory (kStream), the others through its ring (all of them at
+	// once when they fit: then nothing is loaded again)
+	unsigned tmem = 0u;
+	int ntm = 0;
+	if constexpr (kStream) {
+		if (wp == 0) {
+			asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_addr(&tmemBase)), "r"(kTmemCols) : "memory");
+			asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+		}
+		__syncthreads();
+		tmem = tmemBase + ((unsigned) (wp & 3) << 21) + (unsigned) ((wp >> 2) * tmem_slots<B>(pw) * 2 * BB);
+		ntm = min(tmem_slots<B>(pw), wdt);
+		for (int k = 0; k < ntm; ++k) {
+			const int2 *g = (const int2 *) (src + (size_t) (wdt - ntm + k) * kSlot) + lane;
+			int2 e[BB];
+#pragma unroll
+			for (int c = 0; c < B; ++c)
+#pragma unroll
+				for (int r = 0; r < B; ++r) e[c * B + r] = __ldg(g + (r * B + c) * 32);
+			tmem_store<B>(tmem + 2 * BB * k, e);
+		}
+	}
+	const int nring = wdt - ntm, nstage = min(a.stages, nring);
+	const bool stream = kStream && nstage < nring;
+	const int step = kStream ? 1 : a.parts;      // a part's slots: part, part + step, ...
+	if (worker && lane == 0) {
+		for (int k = part; k < nstage; k += step) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(mb + 8 * k) : "memory");
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+		asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+		for (int k = part; k < nstage; k += step) ring_load(ring + k * kSlot, src + (size_t) k * kSlot, kSlot, mb + 8 * k);
+	}
+	int stage = 0, next = nstage;                // ring place of the next slot used, and the next slot to load
+	unsigned parity = 0;
+	// x, p, s and r are used only while the reducer waits for the grid: they stay in global memory (L2), which leaves
+	// the registers to the digit sums; u and the block inverses in shared memory
+	const int vs = nctas * pw * 32 * B, vrow = sl * 32 * B + lane;
+	if (rowWarp) {
+		double *g = a.vec + vrow;
+#pragma unroll
+		for (int c = 0; c < B; ++c) {
+			const long k = (long) i * B + c;
+			g[32 * c] = own ? a.x[k] : 0.0;
+			g[vs + 32 * c] = g[2 * vs + 32 * c] = 0.0;
+			g[3 * vs + 32 * c] = own ? a.r0[k] : 0.0;
+			su[32 * c] = own ? a.u0[k] : 0.0;
+		}
+		double *sbinv = (double *) (sdyn + oInv) + wp * BB * 32 + lane;
+		for (int t = 0; t < BB; ++t) sbinv[32 * t] = own ? __ldg(a.binv + (long) i * BB + t) : 0.0;
+	}
+	const int nst = 32 * (W - 1), nSt = reducer ? 0 : nhalo;    // the reducer warp stages nothing
+	unsigned target = 0;                         // arrivals of the partial-sum path
+	bool pending = false, first = true;
+	int line = 0;                                // sum line of the iteration
+	__syncthreads();
+	if (!stream)
+		for (int k = part; k < nstage; k += step)
+			if (!ring_wait(mb + 8 * k, 0u)) gaveUp = 1;
+	for (;;) {
+		// (0) the halo of u as digits in shared memory
+		// (raw first, in place, for the largest exponent)
+		int e = 1;
+#pragma unroll 4
+		for (int h = threadIdx.x; h < nSt; h += nst) {
+			double v[B];
+			load_halo<B>(a.ug + (long) shalo[h] * U, v);
+			double *d = reinterpret_cast<double *>(slimb + h * S);
+#pragma unroll
+			for (int c = 0; c < B; ++c) { d[c] = v[c]; e = max(e, fx_exp(v[c])); }
+		}
+		e = fx_warp_max(e);
+		if (lane == 0) sE[wp] = e;
+		__syncthreads();
+		const int eU = fx_warp_max(lane < W ? sE[lane] : 1);
+#pragma unroll 1
+		for (int h = threadIdx.x; h < nSt; h += nst) {
+			double *d = reinterpret_cast<double *>(slimb + h * S);
+#pragma unroll
+			for (int c = 0; c < B; ++c) {
+				int2 t;
+				limb_vector(d[c], eU, t.x, t.y);
+				reinterpret_cast<int2 *>(d)[c] = t;
+			}
+		}
+		__syncthreads();
+		// (1) rows: w = A u and (w, u).  Reducer: beta, beta * gamma / alpha and the stopping test of the last update
+		double wv[B], rv[B];
+		double d1 = 0.0;
+#pragma unroll
+		for (int c = 0; c < B; ++c) wv[c] = 0.0;
+		LimbSum acc[B];
+		if (worker) {
+#pragma unroll
+			for (int c = 0; c < B; ++c) acc[c] = limb_zero();
+			if constexpr (kStream) {
+				// tensor-memory slots spread between the streamed ones, which evens out the loads
+				int kt = 0;
+				for (int k = 0; k < nring; ++k) {
+					const int *u = slimb + mycol[k << 5] * S;
+					if (stream && !ring_wait(mb + 8 * stage, parity)) gaveUp = 1;
+					fix_slot_mac<B>(acc, reinterpret_cast<const int2 *>(ring + stage * (int) kSlot) + lane, u);
+					if (stream) {
+						__syncwarp();            // every lane has read the slot before it is overwritten
+						if (lane == 0) ring_load(ring + stage * (int) kSlot, src + next * (int) kSlot, kSlot, mb + 8 * stage);
+						if (++next == nring) next = 0;
+					}
+					if (++stage == nstage) { stage = 0; parity ^= 1u; }
+					if (kt < ntm && (kt + 1) * nring <= (k + 1) * ntm) {
+						int2 e[BB];
+						tmem_load<B>(tmem + 2 * BB * kt, e);
+						tmem_slot_mac<B>(acc, e, slimb + mycol[(nring + kt) << 5] * S);
+						++kt;
+					}
+				}
+				for (; kt < ntm; ++kt) {
+					int2 e[BB];
+					tmem_load<B>(tmem + 2 * BB * kt, e);
+					tmem_slot_mac<B>(acc, e, slimb + mycol[(nring + kt) << 5] * S);
+				}
+			} else {
+				int k = part;
+				for (; k + step < wdt; k += 2 * step) {
+					const int *u = slimb + mycol[k << 5] * S, *u2 = slimb + mycol[(k + step) << 5] * S;
+					fix_slot_mac<B>(acc, reinterpret_cast<const int2 *>(ring + k * (int) kSlot) + lane, u);
+					fix_slot_mac<B>(acc, reinterpret_cast<const int2 *>(ring + (k + step) * (int) kSlot) + lane, u2);
+				}
+				if (k < wdt)
+					fix_slot_mac<B>(acc, reinterpret_cast<const int2 *>(ring + k * (int) kSlot) + lane, slimb + mycol[k << 5] * S);
+				if (part > 0) {
+					long long *o = (long long *) (sdyn + oPart) + ((part - 1) * pw + ws) * 96 * B + lane;
+#pragma unroll
+					for (int c = 0; c < B; ++c) {
+						o[(3 * c) * 32] = acc[c].s2;
+						o[(3 * c + 1) * 32] = acc[c].s1;
+						o[(3 * c + 2) * 32] = acc[c].s0;
+					}
+				}
+			}
+		}
+		if (reducer && pending) {
+			// lanes 0 and 1 share one division: g / gamma and g / alpha
+			const double g = two[0], q = two[1];
+			const double ratio = g / (lane == 1 ? alpha : gam);
+			const double ga = __shfl_sync(0xffffffffu, ratio, 1);
+			if (lane == 0) {
+				beta = ratio;
+				dsub = ratio * ga;
+				gam = g;
+				rr = q;
+				const int n = ++iters;
+				if (fx_exp(g) >= 2047 || fx_exp(q) >= 2047) stop = SA_ERR_NONFINITE;
+				else if (q < goal) stop = SA_OK;
+				else if (n >= itrMax) stop = SA_ERR_NOT_CONVERGED;
+			}
+		}
+		if (!kStream && a.parts > 1 && worker)            // the other parts' digit sums (the reducer is not waited for)
+			asm volatile("bar.sync 1, %0;" :: "r"(32 * pw * a.parts) : "memory");
+		if (rowWarp) {
+			for (int q = 1; !kStream && q < a.parts; ++q) {
+				const long long *o = (const long long *) (sdyn + oPart) + ((q - 1) * pw + ws) * 96 * B + lane;
+#pragma unroll
+				for (int c = 0; c < B; ++c) {
+					acc[c].s2 += o[(3 * c) * 32];
+					acc[c].s1 += o[(3 * c + 1) * 32];
+					acc[c].s0 += o[(3 * c + 2) * 32];
+				}
+			}
+			if (own) {
+#pragma unroll
+				for (int c = 0; c < B; ++c) wv[c] = limb_to_double(acc[c], eRow, eU);
+				d1 = wv[0] * su[0];
+				for (int c = 1; c < B; ++c) d1 += wv[c] * su[32 * c];
+			}
+		}
+		const int fD[1] = {sum_frame(delta)};
+		{
+			const double t[1] = {d1};
+			if (!first) warp_digits<1>(t, fD, dig[wp]);
+		}
+		__syncthreads();                         // digits and scalars
+		if (stop >= 0) break;
+		// (2) reducer: the grid's (w, u) and alpha.  Rows meanwhile: p and s
+		if (reducer && !first) {
+			double t[1];
+			bool flag = false;
+			const bool ok = sum_exchange<1>(dig[0], W, &a.gs->delta[line], nctas, fD, &a.gs->bar, t, flag);
+			if (lc == 0 && lane < kSumWords) a.gs->delta[line >= 1 ? line - 1 : 2].w[lane] = 0ull;
+			if (lane == 0) {
+				if (!ok) gaveUp = 1;
+				slow = flag ? 1 : 0;
+				if (!flag) {
+					delta = t[0];
+					alpha = gam / (t[0] - dsub);
+					// bits, not FP64 compares (64 clocks each): alpha positive and finite, beta finite
+					if (__double_as_longlong(alpha) <= 0 || fx_exp(alpha) >= 2047 || fx_exp(beta) >= 2047)
+						broke = fx_exp(t[0]) < 2047 ? SA_ERR_BREAKDOWN : SA_ERR_NONFINITE;
+				}
+			}
+		} else if (own) {
+			const double be = beta;
+			double *g = a.vec + vs + vrow;
+#pragma unroll
+			for (int c = 0; c < B; ++c) {
+				g[32 * c] = su[32 * c] + be * g[32 * c];
+				wv[c] = wv[c] + be * g[vs + 32 * c];     // s
+				g[vs + 32 * c] = wv[c];
+				rv[c] = g[2 * vs + 32 * c];
+			}
+		}
+		__syncthreads();
+		if (first || slow) {
+			if (!gaveUp && !slow_sum<1>(d1, 0.0, two, a.part, nctas, &a.gs->bar, target, fs)) {
+				if (threadIdx.x == 0) gaveUp = 1;
+			} else if (threadIdx.x == 0 && !gaveUp) {
+				delta = two[0];
+				alpha = gam / (delta - dsub);
+				if (!(alpha > 0.0) || !isfinite(alpha) || !isfinite(beta))
+					broke = isfinite(delta) ? SA_ERR_BREAKDOWN : SA_ERR_NONFINITE;
+			}
+			__syncthreads();
+		}
+		if (gaveUp || broke >= 0) break;
+		const double al = alpha;
+		// (3) rows: r, u and (r, u), (r, r); the reducer adds them over the grid, which also completes u
+		double d2[2] = {0.0, 0.0};
+		if (own) {
+#pragma unroll
+			for (int c = 0; c < B; ++c) rv[c] = rv[c] - al * wv[c];
+			const double *sbinv = (const double *) (sdyn + oInv) + wp * BB * 32 + lane;
+			double uv[B];
+#pragma unroll
+			for (int r = 0; r < B; ++r) {
+				double t = sbinv[32 * (r * B)] * rv[0];
+#pragma unroll
+				for (int c = 1; c < B; ++c) t += sbinv[32 * (r * B + c)] * rv[c];
+				uv[r] = t;
+				su[32 * r] = t;
+			}
+			double2 *o = reinterpret_cast<double2 *>(a.ug + (long) row * U);
+			o[0] = make_double2(uv[0], uv[1]);
+			if constexpr (B == 3) o[1] = make_double2(uv[2], 0.0);
+			d2[0] = rv[0] * uv[0];
+			d2[1] = rv[0] * rv[0];
+			for (int c = 1; c < B; ++c) { d2[0] += rv[c] * uv[c]; d2[1] += rv[c] * rv[c]; }
+		}
+		const int fG[2] = {sum_frame(gam), sum_frame(rr)};
+		warp_digits<2>(d2, fG, dig[wp]);
+		__syncthreads();
+		if (reducer) {
+			double t[2];
+			bool flag = false;
+			__threadfence();                     // the CTA's u before its count
+			const bool ok = sum_exchange<2>(dig[0], W, &a.gs->gamma[line], nctas, fG, &a.gs->bar, t, flag);
+			if (lc == 0 && lane < kSumWords) a.gs->gamma[line >= 1 ? line - 1 : 2].w[lane] = 0ull;
+			if (lane == 0) {
+				if (!ok) gaveUp = 1;
+				slow = flag ? 1 : 0;
+				two[0] = t[0];
+				two[1] = t[1];
+			}
+		} else if (own) {
+#pragma unroll
+			for (int c = 0; c < B; ++c) {                // while the reducer waits
+				double *g = a.vec + vrow + 32 * c;
+				g[0] = g[0] + al * g[vs];
+				g[3 * vs] = rv[c];
+			}
+		}
+		__syncthreads();
+		if (gaveUp) break;
+		if (slow) {
+			if (!slow_sum<2>(d2[0], d2[1], two, a.part + nctas, nctas, &a.gs->bar, target, fs)) {
+				if (threadIdx.x == 0) gaveUp = 1;
+				__syncthreads();
+				break;
+			}
+		}
+		if (++line == 3) line = 0;
+		pending = true;
+		first = false;
+	}
+	if (own)
+#pragma unroll
+		for (int c = 0; c < B; ++c) a.x[(long) i * B + c] = a.vec[vrow + 32 * c];
+	if (stream)                                  // the ring's copies in flight land before the CTA leaves
+		for (int k = 0; k < nstage; ++k) {
+			ring_wait(mb + 8 * stage, parity);
+			if (++stage == nstage) { stage = 0; parity ^= 1u; }
+		}
+	__syncthreads();
+	if constexpr (kStream)
+		if (wp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmemBase), "r"(kTmemCols));
+	if (lc == 0 && threadIdx.x == 0) {
+		sc->iters = iters; sc->code = gaveUp ? SA_ERR_TIMEOUT : max(stop, broke); sc->rr = rr; sc->gam = gam; sc->done = 1;
+	}
+}
+
+template <int B>
+bool cgfix_run(const Mesh &m, const double *blk, const double *binv, double *x, const double *r, const double *u,
+               CgWork &w, cudaEvent_t e0, cudaEvent_t e1, cudaStream_t s)
+{
+	const CgPlan &p = w.plan;
+	if (!p.ok || m.dim != B) return false;
+	static std::mutex mu;
+	static size_t limits[2];
+	static bool known = false;
+	{
+		std::lock_guard<std::mutex> g(mu);
+		if (!known) {
+			limits[0] = fix_smem_limit((const void *) k_cg_fix<B, false>);
+			limits[1] = fix_smem_limit((const void *) k_cg_fix<B, true>);
+			known = true;
+		}
+	}
+	const size_t lim = std::min(limits[0], limits[1]);
+	const int colMax = 32 * p.pw * p.widest;
+	const size_t perStage = (size_t) p.pw * (256 * B * B + 8);
+	const bool resident = fix_smem<B>(p.pw, p.parts, p.haloMax, colMax, p.widest) <= lim;
+	const int parts = resident ? p.parts : 1;
+	const size_t fixed = fix_smem<B>(p.pw, parts, p.haloMax, colMax, 0);
+	if (p.nchunk > kSumMaxCtas || (!resident && fixed + 2 * perStage > lim)) return false;
+	const int stages = resident ? p.widest : (int) ((lim - fixed) / perStage);
+	const size_t smem = fix_smem<B>(p.pw, parts, p.haloMax, colMax, stages);
+	const void *kernel = resident ? (const void *) k_cg_fix<B, false> : (const void *) k_cg_fix<B, true>;
+	int occ = 0;
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 32 * p.warps, smem) != cudaSuccess) {
+		cudaGetLastError();
+		return false;
+	}
+	if (p.nchunk > occ * w.smCount) return false;
+	const int P = p.nchunk * 32 * p.pw;
+	k_cgfix_operator<B><<<(p.nslice + 3) / 4, 128, 0, s>>>(p.nslice, sell_of(m), m.rowPtr, blk, p.perm, p.width, p.off,
+	                                                       p.fix, p.rowExp);
+	k_cgfix_gather_copy<B><<<grid_for(P), kBlock, 0, s>>>(P, p.perm, u, p.ug);
+	SA_CHECK(cudaMemsetAsync(w.bar, 0, sizeof(GridSums), s));
+	FixArgs a{p.pw, parts, p.haloCap, p.haloMax, colMax, stages, p.perm, p.width, p.off, p.halo, p.haloNum, p.rowExp, p.lcol, p.fix,
+	          binv, r, u, x, p.ug, p.vec, w.part, (CgScal *) w.scal, (GridSums *) w.bar};
+	void *args[] = {&a};
+	if (e0) SA_CHECK(cudaEventRecord(e0, s));
+	SA_CHECK(cudaLaunchCooperativeKernel(kernel, dim3(p.nchunk), dim3(32 * p.warps), args, smem, s));
+	if (e1) SA_CHECK(cudaEventRecord(e1, s));
+	w.launches += 3;
+	return true;
+}
+
+template bool cgfix_run<2>(const Mesh &, const double *, const double *, double *, const double *, const double *,
+                           CgWork &, cudaEvent_t, cudaEvent_t, cudaStream_t);
+template bool cgfix_run<3>(const Mesh &, const double *, const double *, double *, const double *, const double *,
+                           CgWork &, cudaEvent_t, cudaEvent_t, cudaStream_t);
+
+}  // namespace sa

@@ -615,6 +615,24 @@ static void alloc_work(Work &w, const Mesh &m, const Model &md, bool wantTraj, P
 	w.trajT = P.zeros<double>((size_t) N * md.timeNum);
 }
 
+// the plan of the fixed-point persistent CG for the FP64 velocity solves of a layered call (none when device memory
+// for it is short: the solves then take the FP64 kernels)
+template <int D>
+static void plan_velocity_cg(Work &w, const Mesh &m, const Model &md, const double *x0soa, Pool &P)
+{
+	if (md.frame || md.ldmWgt != 0.0 || md.precision != SA_PREC_FP64) return;
+	if (md.cgKernel != SA_CG_AUTO && md.cgKernel != SA_CG_PERSISTENT) return;
+	auto alloc = [&](size_t bytes) -> void * {
+		try {
+			return P.alloc<char>(bytes);
+		} catch (const CudaError &) {
+			cudaGetLastError();
+			return nullptr;
+		}
+	};
+	cgfix_plan(m, x0soa, w.cw.smCount, tuning().persistMaxWarps, w.cw.plan, alloc, P.s);
+}
+
 __global__ void k_to_f32(long n, const double *a, float *b)
 {
 	long k = blockIdx.x * (long) blockDim.x + threadIdx.x;
@@ -907,6 +925,7 @@ static int forward_impl(sa_context *ctx, const sa_element_object *obj, const dou
 	std::vector<double> tv = to_host(tauVarMat, (size_t) tauVarNum * objNum, s);
 	Work w;
 	alloc_work<D>(w, m, md, lmkStk != nullptr, P);
+	plan_velocity_cg<D>(w, m, md, x0, P);
 	{   // initial element orientation for the Jacobian sign check
 		double *xa = P.alloc<double>((size_t) m.N * D);
 		launch_soa_to_aos(m.N, D, x0, xa, s);
@@ -1031,6 +1050,7 @@ static int gradient_impl(sa_context *ctx, const sa_element_object *obj, const do
 	const double *tvl = P.dev(tgt->elmVolVec, (size_t) tgt->tgtElmNum);
 	Work w;
 	alloc_work<D>(w, m, md, false, P);
+	plan_velocity_cg<D>(w, m, md, x0, P);
 	{
 		double *xa = P.alloc<double>((size_t) m.N * D);
 		launch_soa_to_aos(m.N, D, x0, xa, s);
@@ -1358,6 +1378,7 @@ static int adjoint_impl(sa_context *ctx, const sa_element_object *obj, const dou
 	const double *tvl = P.dev(tgt->elmVolVec, (size_t) tgt->tgtElmNum);
 	Work w;
 	alloc_work<D>(w, m, md, true, P);
+	plan_velocity_cg<D>(w, m, md, x0, P);
 	const long n = (long) m.N * D, N = m.N;
 	const int T = md.timeNum;
 	const double dt = md.timeStp;
@@ -1543,6 +1564,7 @@ struct Session : SessionBase {
 			tvl = P.dev(tgt->elmVolVec, (size_t) Vt);
 		}
 		alloc_work<D>(w, m, md, false, P);
+		plan_velocity_cg<D>(w, m, md, x0, P);
 		double *xa = P.alloc<double>((size_t) m.N * D);
 		launch_soa_to_aos(m.N, D, x0, xa, s);
 		k_init_sign<D><<<grid_for(m.E), kBlock, 0, s>>>(m.E, m.elmVtx, xa, m.sign0);

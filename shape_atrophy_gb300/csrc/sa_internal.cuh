@@ -14,6 +14,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cfloat>
+#include <functional>
 #include <string>
 #include <vector>
 #include "../../include/shape_atrophy_gb300.h"
@@ -440,7 +441,7 @@ template <int D> void launch_adj_bump_poly(const Mesh &m, const Model &md, const
 // --------------------------------------------------------------------------
 // CG solvers
 // --------------------------------------------------------------------------
-constexpr int kGridBarBytes = 512;   // device memory of the persistent CG's grid barrier
+constexpr int kGridBarBytes = 1280;  // device memory of the persistent CG's grid barrier and sum lines
 
 // Launch shapes chosen by the autotuner (shape_atrophy_gb300/autotune.py, which writes
 // shape_atrophy_gb300/tuning.json; the Python API applies it with sa_set_tuning).  The defaults are the
@@ -455,6 +456,34 @@ struct Tuning {
 	int kernelMatrixFree = 0;      // frame model: 1 = evaluate the RKHS matrix on the fly at every size
 };
 Tuning &tuning();
+
+// device scalars of one CG solve
+struct CgScal {
+	double bb, rr, gam, gamPrev, alpha, beta, delta, tolSqu;
+	int first, done, code, iters, zero, itrMax;
+	unsigned int counter;
+	int pad;
+};
+
+// Row order and column lists of the persistent CG that sums its matrix products in fixed point (sa_limb.cuh).
+// The rows are put in Morton order of the initial node positions and cut into nchunk chunks of at most
+// 32 pw rows, inside a chunk sorted by row length, so that a chunk's rows gather from few distinct nodes (its
+// halo), which its CTA keeps in shared memory.  Permuted row p = chunk * 32 pw + place in the chunk.
+struct CgPlan {
+	bool ok = false;              // built, and every chunk's halo fits
+	int nchunk = 0, pw = 0, warps = 0, nslice = 0, widest = 0, haloCap = 0, haloMax = 0;
+	int parts = 1;                // warps that share a slice's slots (small chunks)
+	long total = 0;               // slots of the permuted sliced layout
+	int *perm = nullptr;          // nchunk 32 pw: node of each permuted row (-1: padding)
+	int *inv = nullptr;           // N: permuted row of each node
+	int *width = nullptr, *off = nullptr;   // nslice (+ 1): longest row and first slot of each 32-row slice
+	unsigned short *lcol = nullptr;         // total: place of each slot's column in its chunk's halo list
+	int *halo = nullptr, *haloNum = nullptr;   // nchunk x haloCap permuted rows, and their count per chunk
+	int2 *fix = nullptr;          // total x B x B: the operator's entries as two digits
+	int *rowExp = nullptr;        // nchunk 32 pw: largest exponent field of each permuted row
+	double *ug = nullptr;         // the gather copy of u in permuted order (3-component nodes padded to 4)
+	double *vec = nullptr;        // x, p, s and r of the permuted rows, [vector][slice][component][lane]
+};
 
 struct CgWork {            // scratch of the Jacobi CG (Chronopoulos-Gear form)
 	double *r, *u, *w, *p, *sv;   // n each
@@ -486,6 +515,7 @@ struct CgWork {            // scratch of the Jacobi CG (Chronopoulos-Gear form)
 	int ctaTabWarps = 0, ctaTabCtas = 0;
 	size_t ctaTabSmem = 0;        // largest column cache of one CTA, bytes
 	std::vector<int> ctaTabHost;
+	CgPlan plan;                  // fixed-point persistent CG (FP64 velocity solves)
 
 	CgWork() = default;
 	CgWork(const CgWork &) = delete;
@@ -497,6 +527,18 @@ struct CgWork {            // scratch of the Jacobi CG (Chronopoulos-Gear form)
 		if (pinned) cudaFreeHost(pinned);
 	}
 };
+
+// fixed-point persistent CG (sa_cgfix.cu): the plan of a mesh (alloc(bytes) returns device memory owned by the
+// caller, or null when there is none), and one solve with r, u and the scalars set by k_cg_init.  cgfix_run
+// returns false when the kernel cannot run (nothing launched).
+bool cgfix_plan(const Mesh &m, const double *x0soa, int smCount, int maxWarps, CgPlan &p,
+                const std::function<void *(size_t)> &alloc, cudaStream_t s);
+template <int B> bool cgfix_run(const Mesh &m, const double *blk, const double *binv, double *x, const double *r,
+                                const double *u, CgWork &w, cudaEvent_t e0, cudaEvent_t e1, cudaStream_t s);
+// Morton order of n points (SoA, D components): sorted 64-bit keys, the point's index in the low 32 bits.
+// scr: morton_order_doubles(D, n) doubles.
+size_t morton_order_doubles(int D, int n);
+template <int D> const unsigned long long *morton_order(int n, const double *soa, double *scr, cudaStream_t s);
 
 template <int B> int cg_jacobi(const Mesh &m, const double *blk, const double *dinv, const double *b,
                                double *x, int itrMax, double tolSqu, CgWork &w, Status *st,

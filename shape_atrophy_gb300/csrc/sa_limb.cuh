@@ -1,0 +1,132 @@
+// sa_limb.cuh -- FP64 products summed on the integer pipes.
+//
+// GB300 issues one FP64 multiply-add per warp every 64 clocks on each SM sub-partition (1.60 per clock per SM
+// measured), but 59 multiply-adds of 32 x 32 -> 64 bit integers per clock per SM.  A sum of products of
+// doubles is therefore formed in fixed point: each factor is cut into signed digits ("limbs") relative to a
+// common power of two, the digit products (at most 2^55) are added in 64-bit integers, which is exact, and the
+// sum is rounded to FP64 once.
+//
+//   matrix entry a of a row whose largest entry has the exponent field eA: va = rint(a 2^(1077 - eA)), |va| <= 2^55,
+//     two digits va = a1 2^28 + a0: exact for entries above a quarter of the row's largest, the others off by at
+//     most 2^-56 of twice the largest (one rounding of an FP64 sum over that row costs 2^-53 of the partial sum);
+//   vector entry u of a set whose largest entry has the exponent field eU: vu = rint(u 2^(1078 - eU)), |vu| <= 2^56,
+//     two digits vu = u1 2^28 + u0: exact for entries above an eighth of the largest, the others off by 2^-57 of
+//     twice it;
+//   sum va vu = 2^56 S2 + 2^28 S1 + S0, S2 = sum a1 u1, S1 = sum (a1 u0 + a0 u1), S0 = sum a0 u0: four integer
+//     multiply-adds per product, nothing dropped.
+// Each sum stays below 2^63 for up to kLimbMaxTerms products.  An Inf or NaN in either factor gives NaN.
+#pragma once
+#include "sa_fixsum.cuh"
+
+namespace sa {
+
+constexpr int kLimbMaxTerms = 120;        // products per sum: 120 x 1.5 x 2^55 < 2^63
+
+// the two digits of a matrix entry in the frame of its row's largest exponent field eA
+SA_FX_HD void limb_matrix(double a, int eA, int &a1, int &a0)
+{
+	int e; unsigned long long m; bool neg;
+	fx_parts(a, e, m, neg);
+	const int d = eA - e;                                     // >= 0
+	const unsigned long long v = d < 64 ? (((m << 3) >> d) + 1ull) >> 1 : 0ull;
+	const long long s = neg ? -(long long) v : (long long) v;
+	const long long lo = ((s + (1ll << 27)) & ((1ll << 28) - 1)) - (1ll << 27);
+	a1 = (int) ((s - lo) >> 28);
+	a0 = (int) lo;
+}
+
+// the two digits of a vector entry in the frame of the set's largest exponent field eU
+SA_FX_HD void limb_vector(double u, int eU, int &u1, int &u0)
+{
+	int e; unsigned long long m; bool neg;
+	fx_parts(u, e, m, neg);
+	const int d = eU - e;                                     // >= 0
+	const unsigned long long v = d < 64 ? (((m << 4) >> d) + 1ull) >> 1 : 0ull;
+	const long long s = neg ? -(long long) v : (long long) v;
+	const int lo = (int) (((unsigned) s + (1u << 27)) & ((1u << 28) - 1u)) - (1 << 27);
+	u1 = (int) ((s - lo) >> 28);
+	u0 = lo;
+}
+
+struct LimbSum { long long s2, s1, s0; };
+
+SA_FX_HD LimbSum limb_zero() { return LimbSum{0ll, 0ll, 0ll}; }
+
+SA_FX_HD void limb_mad(long long &t, int a, int b)
+{
+#if defined(__CUDA_ARCH__)
+	asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(a), "r"(b));
+#else
+	t += (long long) a * b;
+#endif
+}
+
+SA_FX_HD void limb_mac(LimbSum &t, int a1, int a0, int u1, int u0)
+{
+	limb_mad(t.s2, a1, u1);
+	limb_mad(t.s1, a0, u1);
+	limb_mad(t.s1, a1, u0);
+	limb_mad(t.s0, a0, u0);
+}
+
+// v << sh in 128 bits, 0 <= sh < 64
+SA_FX_HD Fx fx_shl(long long v, int sh)
+{
+	return Fx{(unsigned long long) v << sh, sh ? (unsigned long long) (v >> (64 - sh)) : (unsigned long long) (v >> 63)};
+}
+
+SA_FX_HD double limb_bits(unsigned long long bits)
+{
+#if defined(__CUDA_ARCH__)
+	return __longlong_as_double((long long) bits);
+#else
+	double d;
+	__builtin_memcpy(&d, &bits, 8);
+	return d;
+#endif
+}
+
+// results outside the normal range: |value| = f 2^(top - 1150), bit 127 of f set
+SA_FX_HD double limb_edge(Fx f, bool neg, int top)
+{
+	if (top > 2046) return limb_bits((neg ? 1ull << 63 : 0ull) | (2047ull << 52));
+	Fx g{(f.lo >> 1) | (f.hi << 63), f.hi >> 1};              // bit 126: fx_to_double takes signed values
+	if (top < -52) return 0.0;                                // below half the smallest subnormal
+	const double v = fx_to_double(g, top - 14);
+	return neg ? -v : v;
+}
+
+// f 2^(em - 1135) (signed f) as a double, rounded to nearest, ties to even.  One copy for all callers on the device:
+// the solve kernels run their loop body once per iteration, so its length costs instruction fetches.
+#if defined(__CUDACC__)
+static __host__ __device__ __noinline__
+#else
+static
+#endif
+double limb_round(Fx f, int em)
+{
+	const bool neg = (long long) f.hi < 0;
+	if (neg) f = fx_neg(f);
+	int top = em + 15;                                        // exponent field when bit 127 leads
+	if (f.hi == 0ull) { f.hi = f.lo; f.lo = 0ull; top -= 64; }
+	if (f.hi == 0ull) return 0.0;
+	const int z = fx_clz64(f.hi);
+	if (z) { f.hi = (f.hi << z) | (f.lo >> (64 - z)); f.lo <<= z; }
+	top -= z;
+	if (top < 1 || top > 2046) return limb_edge(f, neg, top); // subnormal, or too large
+	// 64 leading bits with the rest as a sticky bit, rounded to 53
+	const unsigned long long q = f.hi >> 11;
+	const unsigned rem = ((unsigned) f.hi & 0x7FFu) | (f.lo ? 1u : 0u);
+	const unsigned long long bits = ((unsigned long long) (top - 1) << 52) + q + (rem + (unsigned) (q & 1ull) > 0x400u ? 1ull : 0ull);
+	return limb_bits(bits | (neg ? 1ull << 63 : 0ull));
+}
+
+// the sum as a double, for the matrix frame eA and the vector frame eU
+SA_FX_HD double limb_to_double(const LimbSum &t, int eA, int eU)
+{
+	if (eA >= 2047 || eU >= 2047) return limb_bits(0x7FF8000000000000ull);     // NaN
+	const Fx f = fx_add(fx_shl(t.s2, 56), fx_add(fx_shl(t.s1, 28), fx_shl(t.s0, 0)));
+	return limb_round(f, eA + eU - 1020);                     // value = f 2^(em - 1135), |f| < 2^120
+}
+
+}  // namespace sa

@@ -521,25 +521,39 @@ static int sort_pad(int n)
 	return p;
 }
 
-// doubles of scratch spatial_order needs for a set of n elements
-static size_t spatial_order_doubles(int D, int n) { return (size_t) (2 * D + 1) * n + sort_pad(n) + 2 * D + 8; }
+size_t morton_order_doubles(int D, int n) { return (size_t) sort_pad(n) + 2 * D + 8; }
 
-// the set S in spatial order, written into scr (spatial_order_doubles(D, S.n) doubles)
 template <int D>
-static VfdSet spatial_order(const VfdSet &S, double *scr, cudaStream_t s)
+const unsigned long long *morton_order(int n, const double *soa, double *scr, cudaStream_t s)
 {
-	if (S.n <= 0) return S;
-	const int n = S.n, npad = sort_pad(n);
-	double *cen = scr, *dir = cen + (long) D * n, *vol = dir + (long) D * n, *box = vol + n;
+	const int npad = sort_pad(n);
+	double *box = scr;
 	unsigned long long *keys = reinterpret_cast<unsigned long long *>(box + 2 * D + 8);
-	k_set_bbox<D><<<1, 256, 0, s>>>(n, S.cen, box);
-	k_set_keys<D><<<(npad + 255) / 256, 256, 0, s>>>(n, npad, S.cen, box, keys);
+	k_set_bbox<D><<<1, 256, 0, s>>>(n, soa, box);
+	k_set_keys<D><<<(npad + 255) / 256, 256, 0, s>>>(n, npad, soa, box, keys);
 	k_bitonic_local<<<npad / kSortBlock, kSortBlock / 2, 0, s>>>(keys, 0);
 	for (int k = 2 * kSortBlock; k <= npad; k <<= 1) {
 		for (int j = k >> 1; j >= kSortBlock; j >>= 1)
 			k_bitonic_global<<<(npad + 255) / 256, 256, 0, s>>>(keys, npad, j, k);
 		k_bitonic_local<<<npad / kSortBlock, kSortBlock / 2, 0, s>>>(keys, k);
 	}
+	return keys;
+}
+
+template const unsigned long long *morton_order<2>(int, const double *, double *, cudaStream_t);
+template const unsigned long long *morton_order<3>(int, const double *, double *, cudaStream_t);
+
+// doubles of scratch spatial_order needs for a set of n elements
+static size_t spatial_order_doubles(int D, int n) { return (size_t) (2 * D + 1) * n + morton_order_doubles(D, n); }
+
+// the set S in spatial order, written into scr (spatial_order_doubles(D, S.n) doubles)
+template <int D>
+static VfdSet spatial_order(const VfdSet &S, double *scr, cudaStream_t s)
+{
+	if (S.n <= 0) return S;
+	const int n = S.n;
+	double *cen = scr, *dir = cen + (long) D * n, *vol = dir + (long) D * n;
+	const unsigned long long *keys = morton_order<D>(n, S.cen, vol + n, s);
 	k_set_gather<D><<<grid_for(n), kBlock, 0, s>>>(n, keys, S, cen, dir, vol);
 	return VfdSet{cen, dir, vol, n};
 }

@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 #pragma unroll
 					for (int c = 0; c < B; ++c) {
 						o[(3 * c) * 32] = acc[c].s2;
-						o[(3 * c + 1) * 32] = acc[c].s1;
+						o[(3 * c + 1) * 32] = acc[c].sm;
 						o[(3 * c + 2) * 32] = acc[c].s0;
 					}
 				}
@@ -600,7 +600,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 #pragma unroll
 				for (int c = 0; c < B; ++c) {
 					acc[c].s2 += o[(3 * c) * 32];
-					acc[c].s1 += o[(3 * c + 1) * 32];
+					acc[c].sm += o[(3 * c + 1) * 32];
 					acc[c].s0 += o[(3 * c + 2) * 32];
 				}
 			}

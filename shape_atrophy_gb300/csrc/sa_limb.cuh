@@ -1,9 +1,9 @@
 // sa_limb.cuh -- FP64 products summed on the integer pipes.
 //
 // GB300 issues one FP64 multiply-add per warp every 64 clocks on each SM sub-partition (1.60 per clock per SM
-// measured), but 59 multiply-adds of 32 x 32 -> 64 bit integers per clock per SM.  A sum of products of
+// measured), but a multiply-add of 32 x 32 -> 64 bit integers in about four.  A sum of products of
 // doubles is therefore formed in fixed point: each factor is cut into signed digits ("limbs") relative to a
-// common power of two, the digit products (at most 2^55) are added in 64-bit integers, which is exact, and the
+// common power of two, the digit products (below 2^57) are added in 64-bit integers, which is exact, and the
 // sum is rounded to FP64 once.
 //
 //   matrix entry a of a row whose largest entry has the exponent field eA: va = rint(a 2^(1077 - eA)), |va| <= 2^55,
@@ -12,15 +12,16 @@
 //   vector entry u of a set whose largest entry has the exponent field eU: vu = rint(u 2^(1078 - eU)), |vu| <= 2^56,
 //     two digits vu = u1 2^28 + u0: exact for entries above an eighth of the largest, the others off by 2^-57 of
 //     twice it;
-//   sum va vu = 2^56 S2 + 2^28 S1 + S0, S2 = sum a1 u1, S1 = sum (a1 u0 + a0 u1), S0 = sum a0 u0: four integer
-//     multiply-adds per product, nothing dropped.
+//   sum va vu = 2^56 S2 + 2^28 S1 + S0, S2 = sum a1 u1, S1 = sum (a1 u0 + a0 u1), S0 = sum a0 u0, nothing dropped.  S1 is
+//     formed as M - S2 - S0 from M = sum (a1 + a0)(u1 + u0) (Karatsuba's product), so a product takes three integer
+//     multiply-adds, each about four clocks of a sub-partition, and two 32-bit additions.
 // Each sum stays below 2^63 for up to kLimbMaxTerms products.  An Inf or NaN in either factor gives NaN.
 #pragma once
 #include "sa_fixsum.cuh"
 
 namespace sa {
 
-constexpr int kLimbMaxTerms = 120;        // products per sum: 120 x 1.5 x 2^55 < 2^63
+constexpr int kLimbMaxTerms = 80;         // products per sum: 80 x 1.5 x 2^56 < 2^63
 
 // the two digits of a matrix entry in the frame of its row's largest exponent field eA
 SA_FX_HD void limb_matrix(double a, int eA, int &a1, int &a0)
@@ -48,7 +49,7 @@ SA_FX_HD void limb_vector(double u, int eU, int &u1, int &u0)
 	u0 = lo;
 }
 
-struct LimbSum { long long s2, s1, s0; };
+struct LimbSum { long long s2, sm, s0; };    // S2, M, S0
 
 SA_FX_HD LimbSum limb_zero() { return LimbSum{0ll, 0ll, 0ll}; }
 
@@ -64,8 +65,7 @@ SA_FX_HD void limb_mad(long long &t, int a, int b)
 SA_FX_HD void limb_mac(LimbSum &t, int a1, int a0, int u1, int u0)
 {
 	limb_mad(t.s2, a1, u1);
-	limb_mad(t.s1, a0, u1);
-	limb_mad(t.s1, a1, u0);
+	limb_mad(t.sm, a1 + a0, u1 + u0);
 	limb_mad(t.s0, a0, u0);
 }
 
@@ -73,6 +73,12 @@ SA_FX_HD void limb_mac(LimbSum &t, int a1, int a0, int u1, int u0)
 SA_FX_HD Fx fx_shl(long long v, int sh)
 {
 	return Fx{(unsigned long long) v << sh, sh ? (unsigned long long) (v >> (64 - sh)) : (unsigned long long) (v >> 63)};
+}
+
+// the sum as one 128-bit integer
+SA_FX_HD Fx limb_fixed(const LimbSum &t)
+{
+	return fx_add(fx_shl(t.s2, 56), fx_add(fx_shl(t.sm - t.s2 - t.s0, 28), fx_shl(t.s0, 0)));
 }
 
 SA_FX_HD double limb_bits(unsigned long long bits)
@@ -125,8 +131,7 @@ double limb_round(Fx f, int em)
 SA_FX_HD double limb_to_double(const LimbSum &t, int eA, int eU)
 {
 	if (eA >= 2047 || eU >= 2047) return limb_bits(0x7FF8000000000000ull);     // NaN
-	const Fx f = fx_add(fx_shl(t.s2, 56), fx_add(fx_shl(t.s1, 28), fx_shl(t.s0, 0)));
-	return limb_round(f, eA + eU - 1020);                     // value = f 2^(em - 1135), |f| < 2^120
+	return limb_round(limb_fixed(t), eA + eU - 1020);         // value = f 2^(em - 1135), |f| < 2^120
 }
 
 }  // namespace sa

@@ -603,11 +603,11 @@ static void alloc_work(Work &w, const Mesh &m, const Model &md, bool wantTraj, P
 		KpcgWork &k = w.kw;
 		k.Ad = P.alloc<double>(n); k.Kid = P.alloc<double>(n); k.r = P.alloc<double>(n);
 		k.Kr = P.alloc<double>(n); k.dv = P.alloc<double>(n); k.wK = P.zeros<double>(n);
-		k.partLen = (long) 4 * nb + 16 * n + 64;
+		k.partLen = std::max(4L * nb + 64, 1024L);             // the launch loop's partials, or 3 per SM
 		k.part = P.alloc<double>((size_t) k.partLen); k.scal = P.zeros<double>(32);
 		k.maxBlocks = nb;
 		k.dv2 = P.alloc<double>(n); k.bar = P.zeros<char>(kGridBarBytes);
-		if (!md.kernelFree) w.K = P.alloc<double>((size_t) N * N);
+		if (!md.kernelFree) w.K = P.alloc<double>(kernel_matrix_entries(m.N));
 	}
 	if (wantTraj) {
 		w.trajX = P.zeros<double>((size_t) n * md.timeNum);

@@ -441,7 +441,7 @@ template <int D> void launch_adj_bump_poly(const Mesh &m, const Model &md, const
 // --------------------------------------------------------------------------
 // CG solvers
 // --------------------------------------------------------------------------
-constexpr int kGridBarBytes = 1280;  // device memory of the persistent CG's grid barrier and sum lines
+constexpr int kGridBarBytes = 1536;  // device memory of the persistent CG's grid barrier and sum lines
 
 // Launch shapes chosen by the autotuner (shape_atrophy_gb300/autotune.py, which writes
 // shape_atrophy_gb300/tuning.json; the Python API applies it with sa_set_tuning).  The defaults are the
@@ -595,6 +595,8 @@ struct KpcgWork {
 // K: the stored kernel matrix, or null to evaluate it on the fly from the node positions q (interleaved)
 template <int D> int kpcg(const Mesh &m, const Model &md, const double *blk, const double *K, const double *q,
                           const double *b, double *x, KpcgWork &w, Status *st, int *itersOut, cudaStream_t s);
+// entries of the stored RKHS matrix (tiled, padded); two 28-bit digits each, the bytes of a double
+size_t kernel_matrix_entries(int N);
 template <int D> void launch_kernel_matrix(const Model &md, int N, const double *x, double *K, cudaStream_t s);
 template <int D> void launch_adj_kernel_term(const Model &md, int N, const double *x, const double *alpha,
                                              const double *beta, double *ax, cudaStream_t s);

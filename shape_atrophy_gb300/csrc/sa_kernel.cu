@@ -17,6 +17,9 @@
 // to the CG tolerance.
 #include "sa_internal.cuh"
 #include "sa_grid.cuh"
+#include "sa_limb.cuh"
+#include <algorithm>
+#include <mutex>
 #include <cmath>
 
 namespace sa {
@@ -213,131 +216,6 @@ __device__ __noinline__ double kernel_entry(int order, double w, Vec<D> qi, Vec<
 	for (int d = 1; d < D; ++d) d2 = d2 + (qi.c[d] - qj.c[d]) * (qi.c[d] - qj.c[d]);
 	return kernel_value<D>(order, w, d2);
 }
-
-// K[j*N + i] = k(|q_i - q_j| / w) + eps * delta_ij
-template <int D>
-__global__ void k_kernel_matrix(int N, const double *__restrict__ x, int order, double w, double eps,
-                                double *__restrict__ K)
-{
-	int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= N) return;
-	const Vec<D> qi = load_node<D>(x, i);
-	for (int j = blockIdx.y; j < N; j += gridDim.y) {
-		double v = kernel_entry<D>(order, w, qi, load_node<D>(x, j));
-		if (i == j) v += eps;
-		K[(long) j * N + i] = v;
-	}
-}
-
-template <int D>
-void launch_kernel_matrix(const Model &md, int N, const double *x, double *K, cudaStream_t s)
-{
-	dim3 g(grid_for(N, 128), std::min(N, 65535));
-	k_kernel_matrix<D><<<g, 128, 0, s>>>(N, x, md.knlOrder, md.knlWidth, md.knlEps, K);
-}
-
-// ---------------------------------------------------------------------------
-// dense K X for D interleaved columns: partial sums over column slices
-// ---------------------------------------------------------------------------
-constexpr int kDenseRows = 128, kDenseSlices = 16, kDenseTile = 128;
-
-template <int D>
-__global__ void k_dense_partial(int N, const double *__restrict__ K, const double *__restrict__ X,
-                                double *__restrict__ part)
-{
-	__shared__ double xs[kDenseTile * D];
-	int i = blockIdx.x * kDenseRows + threadIdx.x;
-	int s = blockIdx.y;
-	int per = (N + kDenseSlices - 1) / kDenseSlices;
-	int j0 = s * per, j1 = min(N, j0 + per);
-	double acc[D];
-	for (int d = 0; d < D; ++d) acc[d] = 0.0;
-	for (int jt = j0; jt < j1; jt += kDenseTile) {
-		int nt = min(kDenseTile, j1 - jt);
-		__syncthreads();
-		for (int t = threadIdx.x; t < nt * D; t += blockDim.x) xs[t] = X[(long) jt * D + t];
-		__syncthreads();
-		if (i < N)
-			for (int jj = 0; jj < nt; ++jj) {
-				double k = K[(long) (jt + jj) * N + i];
-				for (int d = 0; d < D; ++d) acc[d] += k * xs[jj * D + d];
-			}
-	}
-	if (i < N)
-		for (int d = 0; d < D; ++d) part[((long) s * N + i) * D + d] = acc[d];
-}
-
-template <int D>
-__global__ void k_dense_sum(int N, const double *__restrict__ part, double *__restrict__ Y)
-{
-	long k = blockIdx.x * (long) blockDim.x + threadIdx.x;
-	if (k >= (long) N * D) return;
-	double s = 0.0;
-	for (int t = 0; t < kDenseSlices; ++t) s += part[(long) t * N * D + k];
-	Y[k] = s;
-}
-
-template <int D>
-void launch_dense_matvec(int N, const double *K, const double *x, double *y, double *part, cudaStream_t s)
-{
-	dim3 g(grid_for(N, kDenseRows), kDenseSlices);
-	k_dense_partial<D><<<g, kDenseRows, 0, s>>>(N, K, x, part);
-	k_dense_sum<D><<<grid_for((long) N * D), kBlock, 0, s>>>(N, part, y);
-}
-
-// K X without the stored matrix (meshes whose N x N matrix does not fit): the same slices, tiles and
-// summation order as k_dense_partial, each K entry evaluated on the fly by the same kernel_entry as
-// k_kernel_matrix, so the result equals the stored-matrix product bit for bit.  Costs one kernel
-// evaluation (a square root, an exponential, and for 2D Matern the Bessel rational approximations) per
-// matrix entry instead of one 8-byte read.
-template <int D>
-__global__ void k_kernel_partial(int N, const double *__restrict__ q, int order, double w, double eps,
-                                 const double *__restrict__ X, double *__restrict__ part)
-{
-	__shared__ double xs[kDenseTile * D], qs[kDenseTile * D];
-	int i = blockIdx.x * kDenseRows + threadIdx.x;
-	int s = blockIdx.y;
-	int per = (N + kDenseSlices - 1) / kDenseSlices;
-	int j0 = s * per, j1 = min(N, j0 + per);
-	Vec<D> qi;
-	for (int d = 0; d < D; ++d) qi.c[d] = i < N ? q[(long) i * D + d] : 0.0;
-	double acc[D];
-	for (int d = 0; d < D; ++d) acc[d] = 0.0;
-	for (int jt = j0; jt < j1; jt += kDenseTile) {
-		int nt = min(kDenseTile, j1 - jt);
-		__syncthreads();
-		for (int t = threadIdx.x; t < nt * D; t += blockDim.x) {
-			xs[t] = X[(long) jt * D + t];
-			qs[t] = q[(long) jt * D + t];
-		}
-		__syncthreads();
-		if (i < N)
-			for (int jj = 0; jj < nt; ++jj) {
-				Vec<D> qj;
-				for (int d = 0; d < D; ++d) qj.c[d] = qs[jj * D + d];
-				double k = kernel_entry<D>(order, w, qi, qj);
-				if (i == jt + jj) k += eps;
-				for (int d = 0; d < D; ++d) acc[d] += k * xs[jj * D + d];
-			}
-	}
-	if (i < N)
-		for (int d = 0; d < D; ++d) part[((long) s * N + i) * D + d] = acc[d];
-}
-
-// y = K x with K stored (dense) or, when K is null, evaluated from the node positions q
-template <int D>
-static void kernel_matvec(const Model &md, int N, const double *K, const double *q, const double *x, double *y,
-                          double *part, cudaStream_t s)
-{
-	if (K) {
-		launch_dense_matvec<D>(N, K, x, y, part, s);
-		return;
-	}
-	dim3 g(grid_for(N, kDenseRows), kDenseSlices);
-	k_kernel_partial<D><<<g, kDenseRows, 0, s>>>(N, q, md.knlOrder, md.knlWidth, md.knlEps, x, part);
-	k_dense_sum<D><<<grid_for((long) N * D), kBlock, 0, s>>>(N, part, y);
-}
-
 
 // ---------------------------------------------------------------------------
 // K-preconditioned CG (reference ipcg) with device scalars
@@ -545,165 +423,453 @@ __global__ void k_kp_zero(long n, double *x, double *w, const KScal *sc)
 }
 
 // ---------------------------------------------------------------------------
-// Persistent K-preconditioned CG: one cooperative launch runs all iterations of the loop below (six
-// launches per iteration there).  One CTA per SM, kKpWarps warps.  Per iteration three grid-wide exact
-// sums (sa_grid.cuh), which are also the grid's barriers:
-//   A  rows (grid-stride, one thread per row): Kid = r + beta Kid, d = Kr + beta d and
-//      Ad = ldm Kid + (E + btm P) d, with (d, Ad) -> alpha.  A row that gathers a neighbour's d forms it
-//      the same way from the neighbour's previous d and Kr (two d buffers alternate), so no barrier
-//      separates the direction update from the operator;
+// Fixed-point products with the RKHS matrix.  The product with D right-hand sides is N^2 D multiply-adds per
+// iteration, which the FP64 pipe issues at 1.6 per clock per SM: 37 us of a 69 us iteration on the 3131-node strip, where
+// the matrix itself (78 MB) streams from L2 in 5 us.  With the digits below the product takes 20 us there (integer
+// multiply-adds) and the iteration 37 us.  The entries are therefore kept as two 28-bit digits (the bytes
+// of the double; frame: the largest entry, 1 + eps) and multiplied on the integer pipes (sa_limb.cuh); r is converted
+// once per CTA and product into shared memory.  Sums are exact and rounded once, so they do not depend on how rows and
+// columns are dealt out, and the matrix-free form, which converts the same entries on the fly, gives the same bits.
+// ---------------------------------------------------------------------------
+constexpr int kKpWarps = 16;
+constexpr int kKpRows = 8;          // rows of a block: a warp multiplies 8 rows by 4 columns at a time
+constexpr int kKpPass = 4;          // row blocks per pass of a CTA
+constexpr int kKpLoad = 8;          // loads of a thread in flight (matrix entries, entries of r)
+constexpr int kKpFlush = 64;        // products per lane between flushes into 128 bits (kLimbMaxTerms at most)
+static_assert(kKpFlush <= kLimbMaxTerms, "digit sums would overflow");
+
+// the matrix's frame: exponent field of its largest entry
+static int kernel_frame(double eps)
+{
+	const double d = 1.0 + (eps > 0.0 ? eps : 0.0);
+	return fx_exp(d);
+}
+
+// The stored matrix is tiled: 8 rows x 4 columns per 256 bytes, the tiles of a row block one after the other, so that a
+// warp's load is two whole lines and the loads of a batch differ by constants.  Rows and columns past the end hold zero
+// entries.
+__host__ __device__ __forceinline__ int kernel_tiles(int N) { return (N + 3) / 4; }
+__device__ __forceinline__ size_t kernel_place(int N, int i, int j)
+{
+	return ((size_t) (i / kKpRows) * kernel_tiles(N) + j / 4) * 32 + i % kKpRows + kKpRows * (j % 4);
+}
+
+size_t kernel_matrix_entries(int N)
+{
+	return (size_t) ((N + kKpRows - 1) / kKpRows) * kernel_tiles(N) * 32;
+}
+
+// the matrix as digits: one thread per entry on or above the diagonal writes the mirrored entry too (the entries are
+// symmetric bit for bit)
+template <int D>
+__global__ void k_kernel_matrix_fix(int N, const double *__restrict__ x, int order, double w, double eps, int eA,
+                                    int2 *__restrict__ K)
+{
+	const int lane = threadIdx.x & 31, ct = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+	if (ct >= kernel_tiles(N)) return;
+	const int j = 4 * ct + lane / kKpRows;
+	const int nb = (N + kKpRows - 1) / kKpRows;
+	Vec<D> qj;
+	for (int d = 0; d < D; ++d) qj.c[d] = j < N ? x[(long) j * D + d] : 0.0;
+	for (int b = blockIdx.y; b < nb; b += gridDim.y) {
+		const int i = b * kKpRows + lane % kKpRows;
+		if (i >= N || j >= N) {
+			K[((size_t) b * kernel_tiles(N) + ct) * 32 + lane] = make_int2(0, 0);
+			continue;
+		}
+		if (i > j) continue;
+		double v = kernel_entry<D>(order, w, load_node<D>(x, i), qj);
+		if (i == j) v += eps;
+		int2 t;
+		limb_matrix(v, eA, t.x, t.y);
+		K[kernel_place(N, i, j)] = t;
+		K[kernel_place(N, j, i)] = t;
+	}
+}
+
+// a digit sum in 128 bits, moved down to leave room for the sum over up to 2^22 columns of products below 2^111
+constexpr int kKpRoom = 7;
+__device__ __forceinline__ Fx kernel_fixed(const LimbSum &t)
+{
+	const Fx f = limb_fixed(t);
+	return Fx{(f.lo >> kKpRoom) | (f.hi << (64 - kKpRoom)), (unsigned long long) ((long long) f.hi >> kKpRoom)};
+}
+
+__device__ __forceinline__ Fx fx_xor_add(Fx f, int lanes)
+{
+	return fx_add(f, Fx{__shfl_xor_sync(0xffffffffu, f.lo, lanes), __shfl_xor_sync(0xffffffffu, f.hi, lanes)});
+}
+
+template <int D> struct KpSmem {
+	Fx seg[kKpPass][kKpWarps][D][kKpRows];
+	int e[kKpWarps];
+};
+
+// first row block of CTA c: the blocks of kKpRows rows are dealt out evenly and contiguously
+__device__ __forceinline__ int kernel_block0(int N, int c, int nctas)
+{
+	const int nb = (N + kKpRows - 1) / kKpRows;
+	return (int) ((long) nb * c / nctas);
+}
+
+// Kr = K r for the CTA's row blocks [q0, q1): digits of r in shared memory (dig, at most cap nodes at a time, node by node),
+// warp w takes the w-th sixteenth of the columns; lane = row of the block + 8 (column mod 4), so the matrix is read in
+// 64-byte pieces and only two lane exchanges per block add the columns.  out(row, component, value) once per
+// result by one thread.  Every thread of the CTA calls.
+template <int D, bool kFree, typename Out>
+__device__ __forceinline__ void kernel_rows(int N, const int2 *__restrict__ K, const double *__restrict__ q, int order,
+                                            double kw, double eps, int eA, const double *r, int q0, int q1, int2 *dig,
+                                            int cap, KpSmem<D> &sm, Out out)
+{
+	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, W = blockDim.x >> 5;
+	const int nch = (N + cap - 1) / cap;
+	// r (raw, in place of the digits) and its largest exponent.  Each CTA starts at another place: all of them read all of r
+	// right after the barrier, and in step they would queue at one L2 slice after the other
+	double *raw = reinterpret_cast<double *>(dig);
+	int eU = 1;
+	{
+		const int n = min(N, cap) * D, rot = (int) ((unsigned) n * blockIdx.x / gridDim.x);
+		int e = 1;
+		for (int t0 = threadIdx.x; t0 < n; t0 += kKpLoad * blockDim.x) {
+			double v[kKpLoad];                   // all loads before the first store
+#pragma unroll
+			for (int u = 0; u < kKpLoad; ++u) {
+				const int t = t0 + u * blockDim.x, k = t + rot < n ? t + rot : t + rot - n;
+				v[u] = t < n ? __ldcg(r + k) : 0.0;
+			}
+#pragma unroll
+			for (int u = 0; u < kKpLoad; ++u) {
+				const int t = t0 + u * blockDim.x, k = t + rot < n ? t + rot : t + rot - n;
+				if (t < n) raw[k] = v[u];
+				e = max(e, fx_exp(v[u]));
+			}
+		}
+		for (int t = n + threadIdx.x; t < N * D; t += blockDim.x) e = max(e, fx_exp(__ldcg(r + t)));
+		e = fx_warp_max(e);
+		if (lane == 0) sm.e[wp] = e;
+		__syncthreads();
+		eU = fx_warp_max(lane < W ? sm.e[lane] : 1);
+	}
+	for (int p0 = q0; p0 < q1; p0 += kKpPass) {
+		const int nb = min(kKpPass, q1 - p0);
+		for (int c = 0; c < nch; ++c) {
+			const int n0 = c * cap, n = min(N, n0 + cap) - n0;
+			if (nch > 1 || p0 == q0) {           // digits of the chunk's nodes
+				const bool again = nch > 1 && (c > 0 || p0 > q0);
+				if (again) __syncthreads();      // the chunk before has been read
+#pragma unroll 2
+				for (int t = threadIdx.x; t < n * D; t += blockDim.x) {
+					int2 g;
+					limb_vector(again ? __ldcg(r + (long) n0 * D + t) : raw[t], eU, g.x, g.y);
+					dig[t] = g;
+				}
+				__syncthreads();
+			}
+			const int tiles = (n + 3) / 4, t0 = (int) ((unsigned) tiles * wp / W), t1 = (int) ((unsigned) tiles * (wp + 1) / W);
+			// batches of kKpLoad tiles, the next batch's entries loaded (also across row blocks) before a batch is used
+			const int mb = max(1, (t1 - t0 + kKpLoad - 1) / kKpLoad), full = (t1 - t0) / kKpLoad;
+			const int jl = 4 * t0 + (lane >> 3);     // the lane's first column in the chunk
+			int2 ka[kKpLoad], kb[kKpLoad];
+			auto entries = [&](int b, int t, int2 (&k)[kKpLoad]) {
+				if constexpr (kFree) {
+					const int i = (p0 + b) * kKpRows + (lane & 7);
+					const Vec<D> qi = load_node<D>(q, min(i, N - 1));
+#pragma unroll
+					for (int u = 0; u < kKpLoad; ++u) {
+						const int tile = t0 + kKpLoad * t + u, j = n0 + 4 * tile + (lane >> 3);
+						k[u] = make_int2(0, 0);
+						if (tile < t1 && i < N && j < N) {
+							double v = kernel_entry<D>(order, kw, qi, load_node<D>(q, j));
+							if (i == j) v += eps;
+							limb_matrix(v, eA, k[u].x, k[u].y);
+						}
+					}
+				} else {
+					const int2 *p = K + ((size_t) (p0 + b) * kernel_tiles(N) + n0 / 4 + t0 + kKpLoad * t) * 32 + lane;
+#pragma unroll
+					for (int u = 0; u < kKpLoad; ++u) {
+						k[u] = make_int2(0, 0);
+						if (t < full || t0 + kKpLoad * t + u < t1)
+							asm volatile("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(k[u].x), "=r"(k[u].y) : "l"(p + 32 * u));
+					}
+				}
+			};
+			LimbSum acc[D];
+			Fx tot[D];
+			auto use = [&](int b, int t, const int2 (&k)[kKpLoad]) {
+				if (t == 0)
+#pragma unroll
+					for (int d = 0; d < D; ++d) { tot[d] = fx_zero(); acc[d] = limb_zero(); }
+				const int2 *g = dig + (jl + 4 * kKpLoad * t) * D;
+				if (t < full) {
+#pragma unroll
+					for (int u = 0; u < kKpLoad; ++u)
+#pragma unroll
+						for (int d = 0; d < D; ++d) limb_mac(acc[d], k[u].x, k[u].y, g[4 * u * D + d].x, g[4 * u * D + d].y);
+				} else {
+					const int rem = t1 - t0 - kKpLoad * full;
+#pragma unroll
+					for (int u = 0; u < kKpLoad - 1; ++u)
+						if (u < rem)                 // the same for the whole warp
+#pragma unroll
+							for (int d = 0; d < D; ++d) limb_mac(acc[d], k[u].x, k[u].y, g[4 * u * D + d].x, g[4 * u * D + d].y);
+				}
+				const bool last = t == mb - 1;
+				if (last || (t + 1) % (kKpFlush / kKpLoad) == 0)
+#pragma unroll
+					for (int d = 0; d < D; ++d) { tot[d] = fx_add(tot[d], kernel_fixed(acc[d])); acc[d] = limb_zero(); }
+				if (last)
+#pragma unroll
+					for (int d = 0; d < D; ++d) {
+						const Fx s = fx_xor_add(fx_xor_add(tot[d], 8), 16);
+						if (lane < kKpRows) sm.seg[b][wp][d][lane] = c == 0 ? s : fx_add(sm.seg[b][wp][d][lane], s);
+					}
+			};
+			int b = 0, t = 0;
+			auto next = [&](int &bn, int &tn) { if (++tn == mb) { tn = 0; ++bn; } };
+			entries(0, 0, ka);
+			while (b < nb) {
+				int bn = b, tn = t;
+				next(bn, tn);
+				if (bn < nb) entries(bn, tn, kb);
+				use(b, t, ka);
+				b = bn; t = tn;
+				if (b >= nb) break;
+				next(bn, tn);
+				if (bn < nb) entries(bn, tn, ka);
+				use(b, t, kb);
+				b = bn; t = tn;
+			}
+		}
+		__syncthreads();
+		for (int t = threadIdx.x; t < nb * D * kKpRows; t += blockDim.x) {
+			const int a = t % kKpRows, d = t / kKpRows % D, b = t / (kKpRows * D), i = (p0 + b) * kKpRows + a;
+			Fx s = fx_zero();
+#pragma unroll 4
+			for (int g = 0; g < kKpWarps; ++g) s = fx_add(s, sm.seg[b][g][d][a]);
+			const double v = eU >= 2047 || eA >= 2047 ? limb_bits(0x7FF8000000000000ull) : limb_round(s, eA + eU - 1020 + kKpRoom);
+			if (i < N) out(i, d, v);
+		}
+		__syncthreads();
+	}
+}
+
+// y = K x, one launch (the products outside the persistent kernel)
+template <int D, bool kFree>
+__global__ void __launch_bounds__(32 * kKpWarps, 1)
+k_kernel_product(int N, const int2 *__restrict__ K, const double *__restrict__ q, int order, double kw, double eps, int eA,
+                 const double *x, double *y, int cap)
+{
+	extern __shared__ __align__(16) int2 kdig[];
+	__shared__ KpSmem<D> sm;
+	kernel_rows<D, kFree>(N, K, q, order, kw, eps, eA, x, kernel_block0(N, blockIdx.x, gridDim.x),
+	                      kernel_block0(N, blockIdx.x + 1, gridDim.x), kdig, cap, sm,
+	                      [&](int i, int d, double v) { y[(long) i * D + d] = v; });
+}
+
+// ---------------------------------------------------------------------------
+// Persistent K-preconditioned CG: one cooperative launch runs all iterations of the loop below (six launches per
+// iteration there).  One CTA per SM, kKpWarps warps.  Per iteration three grid-wide exact sums that carry the grid's
+// barriers (sum_exchange in sa_grid.cuh; the first iteration, and values that leave their frames, take the partial-sum
+// path):
+//   A  Kid = r + beta Kid, d = Kr + beta d and Ad = ldm Kid + (E + btm P) d, with (d, Ad) -> alpha.  Eight warps share
+//      a slice, each a few of its slots (a row's serial chain of gathers and FP64 operations was 4 us), their partial
+//      products added in a fixed order.  A row that gathers a neighbour's d forms it the same way from the
+//      neighbour's previous d and Kr (two d buffers alternate), so no barrier separates the direction update from
+//      the operator;
 //   B  rows: x += alpha d, w += alpha Kid, r -= alpha Ad, with (r, r) -> stop test;
-//   C  Kr = K r, with (r, Kr) -> beta.  Each CTA forms the whole rows of its row range: K is symmetric bit
-//      for bit (kernel_entry squares differences), so row i is read contiguously, lanes over columns,
-//      warps over (row, column segment) units, a fixed shuffle tree per unit and the segments added in a
-//      fixed order in shared memory.  The matrix-free form evaluates each entry with the same
-//      kernel_entry call the stored matrix was written with, in the same place: both give the same bits.
+//   C  Kr = K r (kernel_rows), with (r, Kr) -> beta.
 // Vectors that other CTAs write during the launch are read with __ldcg (L2), never through the
 // incoherent L1.  Iterates, stopping rule and status codes are those of the loop below.
 // ---------------------------------------------------------------------------
-constexpr int kKpWarps = 16;
-constexpr int kKpUnits = 512;     // (row, segment) units per chunk of phase C
+constexpr int kKpParts = 8;         // warps that share a slice in phase A
+constexpr int kKpGroups = kKpWarps / kKpParts;
 
 struct KpVec {
 	double *x, *w, *r, *Kr, *Kid, *d0, *d1, *Ad;
 };
+
+// sum lines of the three sums (each rotates over three)
+struct KpSums { GridBar bar; SumLine line[3][3]; };
+static_assert(sizeof(KpSums) <= kGridBarBytes, "sum lines larger than their allocation");
 
 __device__ __forceinline__ double kp_dir(double kr, double dOld, double be, bool first)
 {
 	return first ? kr : __fma_rn(be, dOld, kr);
 }
 
+// One grid sum: v summed over all threads of all CTAs; also the grid's barrier (the CTA's writes are visible to the CTAs that
+// passed it).  prev: the sum's value of the iteration before (its frame); slow: no such value yet.  post(sum) runs once per
+// CTA, in one thread, before the CTA goes on: scalar FP64 work in every warp would queue at the FP64 pipe.  false: a wait
+// gave up.
+template <typename Post>
+__device__ __forceinline__ bool kp_sum(double v, double prev, bool slow, int which, int turn, KpSums *ks, double *part,
+                                       unsigned &target, unsigned (*dig)[kSumWords], int *state, FxScratch &fs, Post post)
+{
+	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, W = blockDim.x >> 5, nctas = gridDim.x;
+	bool part_path = slow;
+	if (!slow) {
+		const int frame[1] = {sum_frame(prev)};
+		const double t[1] = {v};
+		warp_digits<1>(t, frame, dig[wp]);
+		__syncthreads();
+		if (wp == 0) {
+			double o[1];
+			bool flag = false;
+			__threadfence();
+			const bool ok = sum_exchange<1>(dig[0], W, &ks->line[which][turn], nctas, frame, &ks->bar, o, flag);
+			if (blockIdx.x == 0 && lane < kSumWords) ks->line[which][turn >= 1 ? turn - 1 : 2].w[lane] = 0ull;
+			if (lane == 0) {
+				*state = ok ? (flag ? 1 : 0) : 2;
+				if (ok && !flag) post(o[0]);
+			}
+		}
+		__syncthreads();
+		if (*state == 2) return false;
+		part_path = *state == 1;
+	}
+	if (part_path) {
+		double a[1] = {v}, o[1];
+		if (!grid_reduce<1, double>(a, o, part + which * nctas, blockIdx.x, nctas, &ks->bar, target, fs)) return false;
+		if (threadIdx.x == 0) post(o[0]);
+		__syncthreads();
+	}
+	return true;
+}
+
+constexpr int kKpColSlots = 4;      // slots of a warp whose columns are kept in shared memory (one slice per warp)
+
 template <int D, bool kFree>
 __global__ void __launch_bounds__(32 * kKpWarps, 1)
-k_kpcg_persist(SellOp A, const double *__restrict__ blk, const double *__restrict__ K, const double *__restrict__ q,
-               int order, double kw, double eps, KpVec v, double *part, KScal *sc, GridBar *bar)
+k_kpcg_persist(SellOp A, const double *__restrict__ blk, const int2 *__restrict__ K, const double *__restrict__ q,
+               int order, double kw, double eps, int eA, KpVec v, double *part, KScal *sc, KpSums *ks, int cap)
 {
+	extern __shared__ __align__(16) int2 kdig[];
 	__shared__ FxScratch fs;
-	__shared__ double segPart[kKpUnits][D];
+	__shared__ KpSmem<D> sm;
+	__shared__ unsigned dig[kKpWarps][kSumWords];
+	__shared__ double apart[kKpWarps][D][32];
+	__shared__ int scol[kKpWarps][kKpColSlots][32];
+	__shared__ double rKr, rr, dAd, alpha, be;
+	__shared__ int sstate, code, it;
 	if (sc->done) return;                       // set before the launch: the same for every CTA
 	const int N = A.N, nctas = gridDim.x, lc = blockIdx.x;
-	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, W = blockDim.x >> 5;
+	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
 	// rows of phases A and B: 32-row slices dealt round-robin over the CTAs first, so that a small mesh
 	// spreads its row work (gathers) over all SMs instead of the first few CTAs
-	const int nsl = (N + 31) >> 5, sl0 = blockIdx.x + gridDim.x * wp, slStride = gridDim.x * W;
-	const double bSqu = sc->bSqu, tolSqu = sc->tolSqu, ldm = sc->ldmWgt;
+	const int nsl = (N + 31) >> 5, grp = wp / kKpParts, prt = wp - grp * kKpParts;
+	const double ldm = sc->ldmWgt;
+	if (threadIdx.x == 0) { rKr = sc->rKr; rr = sc->rSqu; dAd = 0.0; be = 0.0; it = sc->iters; code = -1; }
+	const double goal = sc->bSqu * sc->tolSqu;
 	const int itrMax = sc->itrMax;
-	double rKr = sc->rKr, rr = sc->rSqu, be = 0.0;
-	int it = sc->iters, code = SA_OK;
-	bool first = true;
+	{   // columns of the warp's first slice
+		const int sl = blockIdx.x + gridDim.x * grp;
+		const int w0 = sl < nsl ? __ldg(A.width + sl) : 0;
+		for (int k = prt, t = 0; k < w0 && t < kKpColSlots; k += kKpParts, ++t)
+			scol[wp][t][lane] = __ldg(A.col + __ldg(A.off + sl) + lane + 32 * k);
+	}
+	int turn = 0;
+	bool first = true, ok = true;
 	unsigned int target = 0;
-	double *partA = part, *partB = part + nctas, *partC = part + 2 * nctas;
-	// phase C's row range and (row, segment) units
-	const int r0 = (int) ((long) N * lc / nctas), r1 = (int) ((long) N * (lc + 1) / nctas), R = r1 - r0;
-	const int SEG = min(8, max(1, (2 * W + max(R, 1) - 1) / max(R, 1)));
-	const int RC = kKpUnits / SEG;
+	const int r0 = kernel_block0(N, lc, nctas), r1 = kernel_block0(N, lc + 1, nctas);       // row blocks of phase C
 	double *dOld = v.d0, *dNew = v.d1;
+	__syncthreads();
 	for (;;) {
 		// A: direction, operator, (d, Ad)
-		double loc[1] = {0.0}, res[1];
-		for (int sl = sl0; sl < nsl; sl += slStride) {
-			const int i = sl * 32 + lane, ln = lane;
-			if (i >= N) continue;
-			const int wdt = __ldg(A.width + sl);
-			const long base = __ldg(A.off + sl) + ln;
+		double loc = 0.0;
+		for (int s0 = blockIdx.x; s0 < nsl; s0 += gridDim.x * kKpGroups) {
+			const int sl = s0 + gridDim.x * grp;
+			const double b = be;
 			double acc[D];
 			for (int c = 0; c < D; ++c) acc[c] = 0.0;
-			for (int k = 0; k < wdt; ++k) {
-				const long idx = base + ((long) k << 5);
-				const int j = __ldg(A.col + idx);
-				double dj[D];
-				for (int c = 0; c < D; ++c)
-					dj[c] = kp_dir(__ldcg(v.Kr + (long) j * D + c), first ? 0.0 : __ldcg(dOld + (long) j * D + c),
-					               be, first);
-				double a[D * D];
-				load_block<D, double>(blk, A.total, idx, a);
-				for (int r = 0; r < D; ++r)
-					for (int c = 0; c < D; ++c) acc[r] += a[r * D + c] * dj[c];
+			if (sl < nsl) {
+				const int wdt = __ldg(A.width + sl);
+				const long base = __ldg(A.off + sl) + lane;
+#pragma unroll 2
+				for (int k = prt, t = 0; k < wdt; k += kKpParts, ++t) {
+					const long idx = base + ((long) k << 5);
+					const int j = s0 == (int) blockIdx.x && t < kKpColSlots ? scol[wp][t][lane] : __ldg(A.col + idx);
+					double dj[D];
+					for (int c = 0; c < D; ++c)
+						dj[c] = kp_dir(__ldcg(v.Kr + (long) j * D + c), first ? 0.0 : __ldcg(dOld + (long) j * D + c),
+						               b, first);
+					double a[D * D];
+					load_block<D, double>(blk, A.total, idx, a);
+					for (int r = 0; r < D; ++r)
+						for (int c = 0; c < D; ++c) acc[r] += a[r * D + c] * dj[c];
+				}
 			}
-			for (int c = 0; c < D; ++c) {
-				const long k = (long) i * D + c;
-				const double ri = __ldcg(v.r + k);
-				const double kid = first ? ri : __fma_rn(be, v.Kid[k], ri);
-				const double di = kp_dir(__ldcg(v.Kr + k), first ? 0.0 : __ldcg(dOld + k), be, first);
-				const double ad = __fma_rn(ldm, kid, acc[c]);
+			for (int c = 0; c < D; ++c) apart[wp][c][lane] = acc[c];
+			// one warp per (group, component): its row's vectors meanwhile, then the parts in order
+			const int g = wp / D, c = wp - g * D, slg = s0 + gridDim.x * g, ig = slg * 32 + lane;
+			const bool rows = wp < kKpGroups * D && slg < nsl && ig < N;
+			const long k = (long) ig * D + c;
+			double kid = 0.0, di = 0.0;
+			if (rows) {
+				const double ri = __ldcg(v.r + k), kr = __ldcg(v.Kr + k);
+				const double ko = first ? 0.0 : __ldcg(v.Kid + k), d0 = first ? 0.0 : __ldcg(dOld + k);
+				kid = first ? ri : __fma_rn(b, ko, ri);
+				di = kp_dir(kr, d0, b, first);
 				v.Kid[k] = kid;
 				dNew[k] = di;
+			}
+			__syncthreads();
+			if (rows) {
+				double t = apart[g * kKpParts][c][lane];
+				for (int p = 1; p < kKpParts; ++p) t += apart[g * kKpParts + p][c][lane];
+				const double ad = __fma_rn(ldm, kid, t);
 				v.Ad[k] = ad;
-				loc[0] += di * ad;
+				loc += di * ad;
 			}
+			__syncthreads();
 		}
-		if (!grid_reduce<1, double>(loc, res, partA, lc, nctas, bar, target, fs)) { code = SA_ERR_TIMEOUT; break; }
-		const double dAd = res[0];
-		if (dAd == 0.0 || !isfinite(dAd)) { code = isfinite(dAd) ? SA_ERR_BREAKDOWN : SA_ERR_NONFINITE; break; }
-		const double alpha = rKr / dAd;
-		// B: x, w, r and (r, r)
-		loc[0] = 0.0;
-		for (int sl = sl0; sl < nsl; sl += slStride) {
-			const int i = sl * 32 + lane;
-			if (i >= N) continue;
-			for (int c = 0; c < D; ++c) {
-				const long k = (long) i * D + c;
-				v.x[k] = __fma_rn(alpha, dNew[k], v.x[k]);
-				v.w[k] = __fma_rn(alpha, v.Kid[k], v.w[k]);
-				const double rk = __fma_rn(-alpha, v.Ad[k], v.r[k]);
-				v.r[k] = rk;
-				loc[0] += rk * rk;
-			}
+		ok = kp_sum(loc, dAd, first, 0, turn, ks, part, target, dig, &sstate, fs, [&](double o) {
+			dAd = o;
+			if (o == 0.0 || fx_exp(o) >= 2047) code = o == 0.0 ? SA_ERR_BREAKDOWN : SA_ERR_NONFINITE;
+			alpha = rKr / o;
+		});
+		if (!ok || code >= 0) break;
+		// B: x, w, r and (r, r), one warp per (slice, component) as they were written in A
+		loc = 0.0;
+		const double al = alpha;
+		for (int s0 = blockIdx.x; s0 < nsl; s0 += gridDim.x * kKpGroups) {
+			if (wp >= kKpGroups * D) continue;
+			const int g = wp / D, c = wp - g * D, slg = s0 + gridDim.x * g, ig = slg * 32 + lane;
+			if (slg >= nsl || ig >= N) continue;
+			const long k = (long) ig * D + c;
+			const double x0 = v.x[k], d0 = dNew[k], w0 = v.w[k], k0 = v.Kid[k], a0 = v.Ad[k], q0 = __ldcg(v.r + k);
+			const double rk = __fma_rn(-al, a0, q0);
+			v.r[k] = rk;
+			v.x[k] = __fma_rn(al, d0, x0);
+			v.w[k] = __fma_rn(al, k0, w0);
+			loc += rk * rk;
 		}
-		if (!grid_reduce<1, double>(loc, res, partB, lc, nctas, bar, target, fs)) { code = SA_ERR_TIMEOUT; break; }
-		rr = res[0];
-		++it;
-		if (!isfinite(rr)) { code = SA_ERR_NONFINITE; break; }
-		if (rr < bSqu * tolSqu) { code = SA_OK; break; }
-		if (it >= itrMax) { code = SA_ERR_NOT_CONVERGED; break; }
+		ok = kp_sum(loc, rr, false, 1, turn, ks, part, target, dig, &sstate, fs, [&](double o) {
+			rr = o;
+			const int n = ++it;
+			if (fx_exp(o) >= 2047) code = SA_ERR_NONFINITE;
+			else if (o < goal) code = SA_OK;
+			else if (n >= itrMax) code = SA_ERR_NOT_CONVERGED;
+		});
+		if (!ok || code >= 0) break;
 		// C: Kr = K r over the CTA's rows, (r, Kr)
-		loc[0] = 0.0;
-		for (int c0 = r0; c0 < r1; c0 += RC) {
-			const int rc = min(RC, r1 - c0), units = rc * SEG;
-			for (int u = wp; u < units; u += W) {
-				const int i = c0 + u / SEG, sg = u % SEG;
-				const int j0 = (int) ((long) N * sg / SEG), j1 = (int) ((long) N * (sg + 1) / SEG);
-				double acc[D];
-				for (int c = 0; c < D; ++c) acc[c] = 0.0;
-				Vec<D> qi;
-				if constexpr (kFree) qi = load_node<D>(q, i);
-#pragma unroll 4
-				for (int j = j0 + lane; j < j1; j += 32) {
-					double kij;
-					if constexpr (kFree) {
-						kij = kernel_entry<D>(order, kw, load_node<D>(q, j), qi);   // as K[i N + j] was written
-						if (i == j) kij += eps;
-					} else {
-						kij = __ldg(K + (long) i * N + j);
-					}
-					for (int c = 0; c < D; ++c) acc[c] += kij * __ldcg(v.r + (long) j * D + c);
-				}
-				for (int c = 0; c < D; ++c)
-					for (int off = 16; off > 0; off >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], off);
-				if (lane == 0)
-					for (int c = 0; c < D; ++c) segPart[u][c] = acc[c];
-			}
-			__syncthreads();
-			for (int t = threadIdx.x; t < rc * D; t += blockDim.x) {
-				const int il = t / D, c = t - il * D;
-				double sum = 0.0;
-				for (int sg = 0; sg < SEG; ++sg) sum += segPart[il * SEG + sg][c];
-				const long k = (long) (c0 + il) * D + c;
-				v.Kr[k] = sum;
-				loc[0] += v.r[k] * sum;
-			}
-			__syncthreads();
-		}
-		if (!grid_reduce<1, double>(loc, res, partC, lc, nctas, bar, target, fs)) { code = SA_ERR_TIMEOUT; break; }
-		const double o = res[0];
-		if (o == 0.0 || !isfinite(o)) { code = isfinite(o) ? SA_ERR_BREAKDOWN : SA_ERR_NONFINITE; break; }
-		be = o / rKr;
-		rKr = o;
+		loc = 0.0;
+		kernel_rows<D, kFree>(N, K, q, order, kw, eps, eA, v.r, r0, r1, kdig, cap, sm, [&](int i, int d, double y) {
+			const long k = (long) i * D + d;
+			v.Kr[k] = y;
+			loc += __ldcg(v.r + k) * y;
+		});
+		ok = kp_sum(loc, rKr, false, 2, turn, ks, part, target, dig, &sstate, fs, [&](double o) {
+			if (o == 0.0 || fx_exp(o) >= 2047) code = o == 0.0 ? SA_ERR_BREAKDOWN : SA_ERR_NONFINITE;
+			else { be = o / rKr; rKr = o; }
+		});
+		if (!ok || code >= 0) break;
 		first = false;
+		if (++turn == 3) turn = 0;
 		double *t = dOld; dOld = dNew; dNew = t;
 	}
 	if (lc == 0 && threadIdx.x == 0) {
-		sc->iters = it; sc->code = code; sc->rSqu = rr; sc->rKr = rKr; sc->done = 1;
+		sc->iters = it; sc->code = ok ? code : SA_ERR_TIMEOUT; sc->rSqu = rr; sc->rKr = rKr; sc->done = 1;
 	}
 }
 
@@ -715,30 +881,79 @@ static int device_sm_count()
 	return n;
 }
 
-// one cooperative launch of the persistent K-PCG when every SM can hold one of its CTAs; false: use the loop
+// nodes of r whose digits one CTA holds at a time: all of them up to 160 KB
+constexpr int kKpDigBytes = 160 * 1024;
+template <int D> static int kernel_dig_nodes(int N) { return std::min((N + 3) / 4 * 4, kKpDigBytes / (int) (4 * D * sizeof(int2)) * 4); }
+
+// digits of r in shared memory: the limit of both kernels, raised on first use
 template <int D, bool kFree>
-static bool kpcg_persist_launch(const Mesh &m, const Model &md, const double *blk, const double *K, const double *q,
+static void kp_smem()
+{
+	static std::mutex mu;
+	static bool done = false;
+	std::lock_guard<std::mutex> g(mu);
+	if (done) return;
+	SA_CHECK(cudaFuncSetAttribute(k_kpcg_persist<D, kFree>, cudaFuncAttributeMaxDynamicSharedMemorySize, kKpDigBytes));
+	SA_CHECK(cudaFuncSetAttribute(k_kernel_product<D, kFree>, cudaFuncAttributeMaxDynamicSharedMemorySize, kKpDigBytes));
+	done = true;
+}
+
+// whether the solves of this mesh can run as the persistent K-PCG
+template <int D>
+static bool kpcg_can_persist(const Model &md, int N)
+{
+	if (md.kernelFree) kp_smem<D, true>();
+	else kp_smem<D, false>();
+	if (md.cgKernel == SA_CG_TWO_KERNEL || device_sm_count() > kSumMaxCtas) return false;
+	const size_t bytes = sizeof(int2) * (size_t) D * kernel_dig_nodes<D>(N);
+	int occ = 0;
+	const cudaError_t e = md.kernelFree
+	    ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_kpcg_persist<D, true>, 32 * kKpWarps, bytes)
+	    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_kpcg_persist<D, false>, 32 * kKpWarps, bytes);
+	if (e != cudaSuccess) { cudaGetLastError(); return false; }
+	return occ >= 1;
+}
+
+// one cooperative launch of the persistent K-PCG
+template <int D, bool kFree>
+static void kpcg_persist_launch(const Mesh &m, const Model &md, const double *blk, const int2 *K, const double *q,
                                 double *x, KpcgWork &wk, KScal *sc, cudaStream_t s)
 {
-	int occ = 0;
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_kpcg_persist<D, kFree>, 32 * kKpWarps, 0) !=
-	    cudaSuccess) {
-		cudaGetLastError();
-		return false;
-	}
+	int cap = kernel_dig_nodes<D>(m.N);
+	const size_t bytes = sizeof(int2) * (size_t) D * cap;
 	const int nctas = device_sm_count();
-	if (occ < 1 || 3L * nctas > wk.partLen) return false;
-	GridBar *bar = (GridBar *) wk.bar;
-	SA_CHECK(cudaMemsetAsync(bar, 0, sizeof(GridBar), s));
+	KpSums *ks = (KpSums *) wk.bar;
+	SA_CHECK(cudaMemsetAsync(ks, 0, sizeof(KpSums), s));
 	SellOp A = sell_of(m);
 	KpVec v{x, wk.wK, wk.r, wk.Kr, wk.Kid, wk.dv, wk.dv2, wk.Ad};
-	int order = md.knlOrder;
+	int order = md.knlOrder, eA = kernel_frame(md.knlEps);
 	double kw = md.knlWidth, eps = md.knlEps;
 	double *part = wk.part;
-	void *args[] = {&A, (void *) &blk, (void *) &K, (void *) &q, &order, &kw, &eps, &v, &part, &sc, &bar};
+	void *args[] = {&A, (void *) &blk, (void *) &K, (void *) &q, &order, &kw, &eps, &eA, &v, &part, &sc, &ks, &cap};
 	SA_CHECK(cudaLaunchCooperativeKernel((const void *) k_kpcg_persist<D, kFree>, dim3(nctas), dim3(32 * kKpWarps),
-	                                     args, 0, s));
-	return true;
+	                                     args, bytes, s));
+}
+
+// y = K x with the digit matrix, or evaluated on the fly (K null)
+template <int D>
+static void kernel_product(const Model &md, int N, const int2 *K, const double *q, const double *x, double *y, cudaStream_t s)
+{
+	const int cap = kernel_dig_nodes<D>(N), eA = kernel_frame(md.knlEps);
+	const size_t bytes = sizeof(int2) * (size_t) D * cap;
+	const int nctas = std::min(device_sm_count(), (N + kKpRows - 1) / kKpRows);
+	if (K)
+		k_kernel_product<D, false><<<nctas, 32 * kKpWarps, bytes, s>>>(N, K, q, md.knlOrder, md.knlWidth, md.knlEps, eA, x, y, cap);
+	else
+		k_kernel_product<D, true><<<nctas, 32 * kKpWarps, bytes, s>>>(N, K, q, md.knlOrder, md.knlWidth, md.knlEps, eA, x, y, cap);
+}
+
+// the RKHS matrix of a step, as digits
+template <int D>
+void launch_kernel_matrix(const Model &md, int N, const double *x, double *K, cudaStream_t s)
+{
+	dim3 g(grid_for(kernel_tiles(N), 4), std::min((N + kKpRows - 1) / kKpRows, 65535));
+	k_kernel_matrix_fix<D><<<g, 128, 0, s>>>(N, x, md.knlOrder, md.knlWidth, md.knlEps, kernel_frame(md.knlEps),
+	                                         (int2 *) (void *) K);
 }
 
 template <int D>
@@ -753,23 +968,27 @@ int kpcg(const Mesh &m, const Model &md, const double *blk, const double *K, con
 	h.tolSqu = md.cgTolSqu; h.itrMax = md.cgItrMax; h.ldmWgt = md.ldmWgt;
 	KScal *sc = (KScal *) wk.scal;
 	SA_CHECK(cudaMemcpyAsync(sc, &h, sizeof(KScal), cudaMemcpyHostToDevice, s));
-	double *dpart = wk.part + 4 * (long) nb;     // dense matvec slice partials
+	const int2 *Kfix = (const int2 *) (const void *) K;
+	const bool persist = kpcg_can_persist<D>(md, N);
+	auto product = [&](const double *in, double *out) { kernel_product<D>(md, N, Kfix, q, in, out, s); };
 	k_kp_bnorm<D><<<nb, kKBlock, 0, s>>>(N, b, wk.part, sc);
 	// warm start x0 = K w (w = K^{-1} v of the previous step)
-	kernel_matvec<D>(md, N, K, q, wk.wK, x, dpart, s);
+	product(wk.wK, x);
 	k_kp_init_r<D><<<nb, kKBlock, 0, s>>>(sell_of(m), blk, b, x, wk.wK, wk.r, wk.part, sc);
-	kernel_matvec<D>(md, N, K, q, wk.r, wk.Kr, dpart, s);
+	product(wk.r, wk.Kr);
 	k_kp_rkr<D><<<nb, kKBlock, 0, s>>>(N, wk.r, wk.Kr, wk.part, sc, 1);
 	k_kp_dir<D><<<grid_for(n), kBlock, 0, s>>>(N, wk.r, wk.Kr, wk.Kid, wk.dv, sc, 1);
-	const bool persist = md.cgKernel != SA_CG_TWO_KERNEL && wk.bar && wk.dv2 &&
-	                     (K ? kpcg_persist_launch<D, false>(m, md, blk, K, q, x, wk, sc, s)
-	                        : kpcg_persist_launch<D, true>(m, md, blk, K, q, x, wk, sc, s));
+	SA_CHECK(cudaGetLastError());
+	if (persist) {
+		if (K) kpcg_persist_launch<D, false>(m, md, blk, Kfix, q, x, wk, sc, s);
+		else kpcg_persist_launch<D, true>(m, md, blk, Kfix, q, x, wk, sc, s);
+	}
 	const int chunk = 8;
 	for (int it = 0; !persist && it < md.cgItrMax + chunk; it += chunk) {
 		for (int k = 0; k < chunk; ++k) {
 			k_kp_ad<D><<<nb, kKBlock, 0, s>>>(sell_of(m), blk, wk.dv, wk.Kid, wk.Ad, wk.part, sc);
 			k_kp_step<D><<<nb, kKBlock, 0, s>>>(N, x, wk.wK, wk.r, wk.dv, wk.Kid, wk.Ad, wk.part, sc);
-			kernel_matvec<D>(md, N, K, q, wk.r, wk.Kr, dpart, s);
+			product(wk.r, wk.Kr);
 			k_kp_rkr<D><<<nb, kKBlock, 0, s>>>(N, wk.r, wk.Kr, wk.part, sc, 0);
 			k_kp_dir<D><<<grid_for(n), kBlock, 0, s>>>(N, wk.r, wk.Kr, wk.Kid, wk.dv, sc, 0);
 		}

@@ -272,8 +272,10 @@ __global__ void k_init_sign(int E, const int *__restrict__ elmVtx, const double 
 	sg[e] = det > 0.0 ? 1 : (det < 0.0 ? -1 : 0);
 }
 
+// surfaceOnly: only the boundary elements are needed on the device (varifold).  The element object is checked all the
+// same, on the host, and neither uploaded nor laid out for the solvers; objects in device memory take the full path.
 static void build_mesh(Mesh &m, const sa_element_object *o, bool needVfd, bool needGrad, bool layered, int lyrNum,
-                       Pool &P, PhaseTrace *tr = nullptr)
+                       Pool &P, PhaseTrace *tr = nullptr, bool surfaceOnly = false)
 {
 	cudaStream_t s = P.s;
 	int D = o->dim;
@@ -289,19 +291,25 @@ static void build_mesh(Mesh &m, const sa_element_object *o, bool needVfd, bool n
 	SA_REQUIRE((long) m.E * 16 < (1L << 31), "too many elements for the 32-bit assembly table");
 	m.vtxElmCols = o->vtxElmCols; m.femIfoCols = o->femIfoCols;
 	int frmCols = D == 2 ? 4 : 6;
-	m.elmVtx = (int *) P.dev(o->elmVtxMat, (size_t) m.E * m.V);
-	m.vtxElm = (int *) P.dev(o->vtxElmMat, (size_t) m.N * o->vtxElmCols);
-	if (haveFrame) {
-		m.frmVtx = (int *) P.dev(o->frmVtxMat, (size_t) m.E * frmCols);
-		m.tsvVtx = (int *) P.dev(o->tsvVtxMat, (size_t) m.E * frmCols);
+	for (const int *p : {o->elmVtxMat, o->vtxElmMat, o->frmVtxMat, o->tsvVtxMat, o->femVtxMat, o->femIfoMat, o->btmVtxMat, o->vtxBtmMat})
+		surfaceOnly = surfaceOnly && !is_device_ptr(p);
+	if (!surfaceOnly) {
+		m.elmVtx = (int *) P.dev(o->elmVtxMat, (size_t) m.E * m.V);
+		m.vtxElm = (int *) P.dev(o->vtxElmMat, (size_t) m.N * o->vtxElmCols);
+		if (haveFrame) {
+			m.frmVtx = (int *) P.dev(o->frmVtxMat, (size_t) m.E * frmCols);
+			m.tsvVtx = (int *) P.dev(o->tsvVtxMat, (size_t) m.E * frmCols);
+		}
+		m.femVtx = (int *) P.dev(o->femVtxMat, (size_t) m.Z * 2);
+		m.femIfo = (int *) P.dev(o->femIfoMat, (size_t) m.Z * o->femIfoCols);
 	}
-	m.femVtx = (int *) P.dev(o->femVtxMat, (size_t) m.Z * 2);
-	m.femIfo = (int *) P.dev(o->femIfoMat, (size_t) m.Z * o->femIfoCols);
 	if (m.Bt > 0) {
 		SA_REQUIRE(o->btmVtxMat && o->vtxBtmMat && o->vtxBtmCols >= 1 && m.Nb > 0 && m.Nb <= m.N,
 		           "bottom arrays inconsistent");
-		m.btmVtx = (int *) P.dev(o->btmVtxMat, (size_t) m.Bt * D);
-		m.vtxBtm = (int *) P.dev(o->vtxBtmMat, (size_t) m.Nb * o->vtxBtmCols);
+		if (!surfaceOnly) {
+			m.btmVtx = (int *) P.dev(o->btmVtxMat, (size_t) m.Bt * D);
+			m.vtxBtm = (int *) P.dev(o->vtxBtmMat, (size_t) m.Nb * o->vtxBtmCols);
+		}
 		m.vtxBtmCols = o->vtxBtmCols;
 	}
 	if (needVfd) {
@@ -433,6 +441,39 @@ static void build_mesh(Mesh &m, const sa_element_object *o, bool needVfd, bool n
 		         "elmLyrVec entry outside the layer tables");
 	}
 	if (tr) tr->mark("mesh: validate");
+	if (surfaceOnly) {
+		// the checks that the layout and the assembly table below make
+		long total = 0;
+		for (int sl = 0; 32L * sl < m.N; ++sl) {
+			int w = 0;
+			for (int i = 32 * sl; i < std::min(m.N, 32 * sl + 32); ++i) w = std::max(w, rp[i + 1] - rp[i]);
+			total += 32L * w;
+		}
+		SA_REQUIRE(total < (1L << 31) / 8, "operator too large for 32-bit slot offsets");
+		parallel_chunks(m.Z, [&](long lo, long up) {
+			for (long z = lo; z < up; ++z) {
+				const int i = fv[z], j = fv[m.Z + z];
+				const int *b = fv + m.Z + rp[j], *e = fv + m.Z + rp[j + 1];
+				const int *q = std::lower_bound(b, e, i);
+				SA_REQUIRE(q != e && *q == i, "femVtxMat pattern is not symmetric");
+				SA_REQUIRE(fi[z] == fi[rp[j] + (int) (q - b)], "femIfoMat lists differ between (i, j) and (j, i)");
+			}
+		});
+		const int *ifo = o->femIfoMat;
+		parallel_chunks(m.Z, [&](long lo, long up) {
+			for (long z = lo; z < up; ++z)
+				for (int k = 0; k < fi[z]; ++k) {
+					const int e = ifo[(2 + 2 * k) * (long) m.Z + z];
+					bool a = false, b = false;
+					for (int l = 0; e >= 0 && e < m.E && l < m.V; ++l) {
+						a = a || ev[(long) l * m.E + e] == fv[z];
+						b = b || ev[(long) l * m.E + e] == fv[m.Z + z];
+					}
+					SA_REQUIRE(a && b, "femIfoMat lists an element that does not contain both nodes of the slot");
+				}
+		});
+		return;
+	}
 	m.rowPtr = P.alloc<int>(m.N + 1);
 	SA_CHECK(cudaMemcpyAsync(m.rowPtr, rp.data(), sizeof(int) * (m.N + 1), cudaMemcpyHostToDevice, s));
 	{   // sliced layout: 32-row slices, slot k of row 32 s + lane at off[s] + 32 k + lane
@@ -983,7 +1024,7 @@ static int varifold_impl(sa_context *ctx, const sa_element_object *obj, const do
                          int precision, double *objOut, double *grad)
 {
 	cudaStream_t s = ctx->stream;
-	Pool P(s);
+	Pool P(s, true);
 	Mesh m;
 	Model md;
 	memset(&md, 0, sizeof(md));
@@ -996,7 +1037,7 @@ static int varifold_impl(sa_context *ctx, const sa_element_object *obj, const do
 	           "dirKnlType must be B, L, O or U");
 	SA_REQUIRE(kernel_widths_ok(md.cenWidth, md.dirKnl, md.dirWidth),
 	           "cenKnlWidth (and dirKnlWidth for 'O'/'U') must be finite and > 0");
-	build_mesh(m, obj, true, grad != nullptr, false, 0, P);
+	build_mesh(m, obj, true, grad != nullptr, false, 0, P, nullptr, true);
 	const double *x = P.dev(lmk, (size_t) m.N * D);
 	double *xa = P.alloc<double>((size_t) m.N * D);
 	launch_soa_to_aos(m.N, D, x, xa, s);
@@ -1009,11 +1050,9 @@ static int varifold_impl(sa_context *ctx, const sa_element_object *obj, const do
 	SA_REQUIRE(err == SA_OK, "varifold gradient needs vfdIfoMat");
 	*objOut = v;
 	if (grad) {
-		// back to the reference's column-major N x D layout
-		std::vector<double> h = to_host(ga, (size_t) m.N * D, s), o((size_t) m.N * D);
-		for (int i = 0; i < m.N; ++i)
-			for (int d = 0; d < D; ++d) o[(size_t) d * m.N + i] = h[(size_t) i * D + d];
-		SA_CHECK(cudaMemcpyAsync(grad, o.data(), sizeof(double) * o.size(), cudaMemcpyDefault, s));
+		// back to the reference's column-major N x D layout (the interleaved copy of x is free by now)
+		launch_aos_to_soa(m.N, D, ga, xa, s);
+		SA_CHECK(cudaMemcpyAsync(grad, xa, sizeof(double) * m.N * D, cudaMemcpyDefault, s));
 		SA_CHECK(cudaStreamSynchronize(s));
 	}
 	return SA_OK;

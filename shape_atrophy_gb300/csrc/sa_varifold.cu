@@ -143,6 +143,18 @@ __device__ __forceinline__ double sqrt_nr(double a)
 	return s;
 }
 
+// 1 / a for a >= 1 in FP64 by Newton's iteration y <- y + y (1 - a y) from the FP32 reciprocal (relative error a few
+// 1e-8, squared by each of the two steps): four FP64 multiply-adds and two conversions instead of a division.
+// Arguments of 2^96 and above (and NaN) are divided.
+__device__ __forceinline__ double rcp_nr(double a)
+{
+	if ((unsigned) __double2hiint(a) >= (1023u + 96u) << 20) return 1.0 / a;
+	double y = (double) (1.0f / __double2float_rn(a));
+	y = fma(y, fma(-a, y, 1.0), y);
+	return fma(y, fma(-a, y, 1.0), y);
+}
+__device__ __forceinline__ float rcp_nr(float a) { return 1.0f / a; }
+
 __device__ __forceinline__ double exp_k(double x, const double *tab) { return exp_tab(x, tab); }
 __device__ __forceinline__ float exp_k(float x, const double *) { return exp(x); }
 __device__ __forceinline__ double sqrt_k(double x) { return sqrt_nr(x); }
@@ -166,7 +178,7 @@ template <typename T>
 __device__ __forceinline__ T cen_knl_scaled(int type, T d2, const double *tab)
 {
 	if (type == 'G') return exp_k(-d2, tab);
-	if (type == 'C') return (T) 1.0 / ((T) 1.0 + d2);
+	if (type == 'C') return rcp_nr((T) 1.0 + d2);
 	T r = sqrt_k(d2), ex = exp_k(-r, tab);          // 'M'
 	return fma(r, ex, ex);
 }
@@ -180,6 +192,20 @@ __device__ __forceinline__ T dir_knl(int type, T iw2, T ang, T &d1, const double
 	T k = exp_k((T) 2.0 * (ang * ang - (T) 1.0) * iw2, tab);     // 'U'
 	if (G) d1 = (T) 4.0 * ang * k * iw2;
 	return k;
+}
+
+// The gradient rows' FP64 work per pair is what bounds them (5120 x 5120 triangles, 'C' x 'O': 12.1 -> 7.2 ms a call when
+// the divisions, the width scalings and the row factors left the pair loop).
+// Kernel values of the gradient rows for centres multiplied by 1/w (c'), with the part of the derivative that varies
+// with the pair: dK/dc' = f cg (c_i' - c_j'), cg = K ('G'), K^2 ('C'), e^-r ('M'), f = -2, -2, -1
+template <typename T>
+__device__ __forceinline__ T cen_knl_grad(int type, T d2, T &cg, const double *tab)
+{
+	if (type == 'G') return cg = exp_k(-d2, tab);
+	if (type == 'C') { const T k = rcp_nr((T) 1.0 + d2); cg = k * k; return k; }
+	T r = sqrt_k(d2), ex = exp_k(-r, tab);
+	cg = ex;
+	return fma(r, ex, ex);
 }
 
 // exp_tab and exp() (fn 0) or sqrt_nr and sqrt() (fn 1) side by side: accuracy check
@@ -250,9 +276,9 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 	// cancellation DD - 2 DT + TT).
 	constexpr bool kNear = kSplit && !G;
 	constexpr int kN = kNear ? 1 : 0;
-	// FP64 objective: centres (rows and tiles) multiplied by 1/w as they are loaded, so the pair term does
-	// not scale the squared distance (the gradient keeps unscaled centres for its derivatives)
-	constexpr bool kScaled = !kSplit && !G;
+	// FP64: centres (rows and tiles) multiplied by 1/w as they are loaded, so the pair term does not scale the squared
+	// distance (the gradient's centre derivatives are multiplied by 1/w once per row)
+	constexpr bool kScaled = !kSplit;
 	const double cs = kScaled ? 1.0 / cw : 1.0;
 	__shared__ T sc[kVfdTile * D], su[kVfdTile * D], sv[kVfdTile], sl[kSplit ? kVfdTile * D : 1];
 	__shared__ double sc64[kN * kVfdTile * D + 1], su64[kN * kVfdTile * D + 1], sv64[kN * kVfdTile + 1];
@@ -331,7 +357,7 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 			// tile = sum of K_c K_d vol_j over the tile's columns; the row factor coef * vol_i and, for the
 			// symmetric half, the weights (2 off the diagonal, 1 on it: 2 tile - diagonal term) are applied
 			// once per tile
-			T tile = 0, comp = 0, diag = 0, tgc[D], tgt[D];
+			T tile = 0, comp = 0, diag = 0, angSum = 0, tgc[D], tgt[D];
 			double nearSum = 0.0, diag64 = 0.0;                       // FP64 near-field terms (kNear)
 			for (int d = 0; d < D; ++d) { tgc[d] = 0; tgt[d] = 0; }
 			for (int jj = 0; jj < nt; ++jj) {
@@ -351,9 +377,23 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 				T ang = ui[0] * su[jj * D];
 				for (int d = 1; d < D; ++d) ang = ang + ui[d] * su[jj * D + d];
 				T d1c = 0, d1d = 0;
+				T vj = sv[jj];
+				if constexpr (kScaled && G) {
+					// per pair: t = K_c K_d v_j; centre part cg K_d v_j df; direction part b u_j with b = K_c K_d' v_j, and
+					// the row's own direction with weight t - b ang, i.e. tile - angSum at the end of the tile
+					T cg;
+					const T kc = cen_knl_grad<T>(ck, d2, cg, sExp), kd = dir_knl<T, true>(dk, diw2, ang, d1d, sExp);
+					const T kv = kc * vj, cv = ck == 'G' ? kv * kd : (cg * vj) * kd, b = kv * d1d;
+					tile = fma(kv, kd, tile);
+					angSum = fma(b, ang, angSum);
+					for (int d = 0; d < D; ++d) {
+						tgc[d] = fma(cv, df[d], tgc[d]);
+						tgt[d] = fma(b, su[jj * D + d], tgt[d]);
+					}
+					continue;
+				}
 				T kc = kScaled ? cen_knl_scaled<T>(ck, d2, sExp) : cen_knl<T, G>(ck, ciw, ciw2, d2, d1c, sExp);
 				T kd = dir_knl<T, G>(dk, diw2, ang, d1d, sExp);
-				T vj = sv[jj];
 				const T kv = kd * vj;
 				if (kNear && kc * kd > (T) kNearField) {
 					double e2 = 0.0, a64 = 0.0, u1 = 0.0, u2 = 0.0;
@@ -388,7 +428,16 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 			// Kahan: the FP32 sum with its lost low part, plus the FP64 near-field terms
 			const double tsum = ((double) tile - (double) comp) + nearSum;
 			acc += cv * (sym ? 2.0 * tsum - ((double) diag + diag64) : tsum);
-			if (G) for (int d = 0; d < D; ++d) { gc[d] += (double) tgc[d]; gt[d] += (double) tgt[d]; }
+			if (kScaled && G) {
+				// centre part times f / w and the row's weights (cen_knl_grad); directions: D = 2: v = |e|, D = 3: v = |n| / 2
+				const double fc = (double) gco * (double) vi * cs * (ck == 'M' ? -1.0 : -2.0), ft = (double) gco * (double) half;
+				for (int d = 0; d < D; ++d) {
+					gc[d] += fc * (double) tgc[d];
+					gt[d] += ft * ((double) tgt[d] + (double) ui[d] * ((double) tile - (double) angSum));
+				}
+			} else if (G) {
+				for (int d = 0; d < D; ++d) { gc[d] += (double) tgc[d]; gt[d] += (double) tgt[d]; }
+			}
 		}
 	}
 	if (act) {

@@ -730,7 +730,10 @@ static void launch_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet B, double cB, 
 }
 
 // column chunks of the pair sums of a Vd x Vt objective: enough CTAs to fill the GPU (the pair sums are latency
-// bound at one CTA per SM), each chunk at least two tiles wide
+// bound at one CTA per SM), each chunk at least kVfdMinCols columns wide.  A warp alone on its sub-partition issues an
+// FP64 operation every 64 clocks whatever the chunk, so small sets want many narrow chunks: 512 x 512 segments with
+// gradient, 256 columns per chunk 0.9 ms in the pair sums, 16 columns 0.1 ms.
+constexpr int kVfdMinCols = 16;
 int vfd_chunk_count(int Vd, int Vt)
 {
 	int dev = 0, sms = 1;
@@ -740,7 +743,7 @@ int vfd_chunk_count(int Vd, int Vt)
 	const int perSm = std::max(1, tuning().vfdCtasPerSm);
 	const int rowCtas = std::max(1, grid_for(rowMax, kVfdBlock));
 	int C = std::max(1, (perSm * sms + rowCtas - 1) / rowCtas);
-	C = std::min(C, std::max(1, colMin / (2 * kVfdTile)));
+	C = std::min(C, std::max(1, colMin / kVfdMinCols));
 	return std::min(C, 32);
 }
 

@@ -28,6 +28,7 @@ constexpr int kFixMaxWarps = 20;           // CTA size limit, reducer warp inclu
 constexpr int kFixMinWarps = 8;            // small solves: warps without rows help to stage the halo
 constexpr int kFixMaxParts = 8;            // warps per slice
 constexpr int kFixMaxHalo = 8192;          // halo nodes per chunk (shared memory takes about 6000 of them)
+constexpr int kFixStagers = 4;             // warps that stage at least, with several chunks per CTA
 constexpr int kFixMaxRows = 1 << 20;       // permuted rows whose bit map and prefix counts fit shared memory
 
 template <int B> constexpr int limb_stride() { return 6; }    // words per halo node: three 8-byte bank pairs, odd, so consecutive nodes spread
@@ -165,14 +166,21 @@ bool cgfix_plan(const Mesh &m, const double *x0soa, int smCount, int maxWarps, C
 	const int cap = std::min(kFixMaxWarps, maxWarps) - 1;
 	if (cap < 1 || smCount < 1) return false;
 	p.pw = std::max(1, (ns0 + smCount - 1) / smCount);
-	if (p.pw > cap) return false;
+	p.per = 1;
 	p.nchunk = (ns0 + p.pw - 1) / p.pw;
+	if (p.pw > cap) {                            // several chunks per CTA, and warps that stage the next chunk
+		const int rows = cap - kFixStagers;
+		if (rows < 1) return false;
+		p.per = (ns0 + rows * smCount - 1) / (rows * smCount);
+		p.nchunk = p.per * smCount;
+		p.pw = (ns0 + p.nchunk - 1) / p.nchunk;
+	}
 	for (size_t q = 0; q + 1 < m.slOffHost.size(); ++q)
 		p.widest = std::max(p.widest, (m.slOffHost[q + 1] - m.slOffHost[q]) / 32);
 	// small chunks: several warps share a slice, two slots or more each (a slot costs one warp about 450 clocks of
 	// latency, against 160 of issue; the digit sums are integers, so the split changes no bit)
-	p.parts = std::max(1, std::min({cap / p.pw, kFixMaxParts, (p.widest + 1) / 2}));
-	p.warps = std::max(std::min(kFixMinWarps, maxWarps), p.pw * p.parts + 1);
+	p.parts = p.per > 1 ? 1 : std::max(1, std::min({cap / p.pw, kFixMaxParts, (p.widest + 1) / 2}));
+	p.warps = p.per > 1 ? cap + 1 : std::max(std::min(kFixMinWarps, maxWarps), p.pw * p.parts + 1);
 	p.nslice = p.nchunk * p.pw;
 	p.haloCap = std::min(kFixMaxHalo, p.nchunk * 32 * p.pw);
 	const int R = 32 * p.pw, P = p.nchunk * R;
@@ -198,7 +206,8 @@ bool cgfix_plan(const Mesh &m, const double *x0soa, int smCount, int maxWarps, C
 	p.rowExp = (int *) get(sizeof(int) * (size_t) P);
 	p.ug = (double *) get(sizeof(double) * (size_t) P * (B == 3 ? fix_u_stride<3>() : fix_u_stride<2>()));
 	p.vec = (double *) get(sizeof(double) * (size_t) P * 4 * B);
-	if (!p.lcol || !p.fix || !p.rowExp || !p.ug || !p.vec) return false;
+	if (p.per > 1) p.pinv = (double *) get(sizeof(double) * (size_t) P * B * B);
+	if (!p.lcol || !p.fix || !p.rowExp || !p.ug || !p.vec || (p.per > 1 && !p.pinv)) return false;
 	const int nw = (P + 31) / 32;
 	const size_t sm = sizeof(int) * (size_t) nw + sizeof(unsigned short) * (size_t) (nw + 1);
 	if (sm > 48 * 1024 && sm > fix_smem_limit((const void *) k_plan_columns)) return false;
@@ -261,7 +270,7 @@ struct FixArgs {
 	const unsigned short *lcol;
 	const int2 *fix;
 	const double *binv, *r0, *u0;
-	double *x, *ug, *vec, *part;
+	double *x, *ug, *vec, *part, *pinv;
 	CgScal *sc;
 	GridSums *gs;
 };
@@ -276,11 +285,23 @@ template <int B> size_t fix_smem(int pw, int parts, int haloMax, int colMax, int
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned) __cvta_generic_to_shared(p); }
 
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, unsigned bar)
+{
+	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+	             :: "r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+// the same with an L2 policy
+__device__ __forceinline__ void bulk_load_hint(void *dst, const void *src, unsigned bytes, unsigned bar, unsigned long long policy)
+{
+	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+	             :: "r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(bar), "l"(policy) : "memory");
+}
+
 __device__ __forceinline__ void ring_load(void *dst, const void *src, unsigned bytes, unsigned bar)
 {
 	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
-	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-	             :: "r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(bar) : "memory");
+	bulk_load(dst, src, bytes, bar);
 }
 
 constexpr int kRingTries = 1 << 20;        // bounded wait: each try suspends up to a hardware time limit
@@ -734,6 +755,387 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 	}
 }
 
+// ---------------------------------------------------------------------------
+// The same solve for operators of more than one chunk per CTA (97 000 nodes and up).  The CTA takes its per chunks in
+// turn: the row warps multiply one while the staging warps gather and convert the next one's halo.  The warp's operator
+// ring, whose slots carry their columns, runs on from chunk to chunk; the last slots of the first chunk's slices stay in
+// tensor memory.  x, p, s and r of the rows and their block inverses are in global memory, 32 rows of a component together
+// (72 bytes a row in the natural order cost 9 x 32 cache tags per slice, 10k clocks of an iteration).
+//
+// What bounds it: the operator's bytes.  At 204 810 nodes (3 chunks of 15 slices, 215 MB of entries and columns, 182 of
+// them through the ring) 70 of an iteration's 113 thousand clocks are the products, 5.3 TB/s; the rest is the rows' FP64
+// (16k), the two grid sums (15k) and the first halo (6k).  A solve of it: 81 us per iteration in the FP64 kernel, 85 with
+// each chunk staged by the warps that multiply it, 60 with staging warps and columns in the ring, 55 with the ring's loads
+// marked evict-first (a kept first chunk, or two, gave nothing more).
+// ---------------------------------------------------------------------------
+template <int B>
+__global__ void k_cgfix_inverses(int P, const int *__restrict__ perm, const double *__restrict__ binv, double *__restrict__ out)
+{
+	const int q = blockIdx.x * blockDim.x + threadIdx.x;
+	if (q >= P) return;
+	const int i = perm[q];
+	for (int t = 0; t < B * B; ++t)
+		out[(long) (q >> 5) * (32 * B * B) + 32 * t + (q & 31)] = i >= 0 ? binv[(long) i * (B * B) + t] : 0.0;
+}
+
+// bytes of a ring slot: entries and columns
+template <int B> __host__ __device__ constexpr int many_slot() { return 256 * B * B + 64; }
+
+// shared memory: operator ring and its barriers, two chunks' halo digits, the first chunk's halo rows, columns of the
+// slots in tensor memory
+template <int B> size_t fix_many_smem(int pw, int haloMax, int stages)
+{
+	return (size_t) pw * stages * (many_slot<B>() + 8) + sizeof(int) * (size_t) haloMax * (2 * limb_stride<B>() + 1) +
+	       (size_t) pw * tmem_slots<B>(pw) * 64 + 16;
+}
+
+template <int B>
+__global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix_many(const FixArgs a, int per)
+{
+	__shared__ FxScratch fs;
+	__shared__ unsigned dig[kFixMaxWarps][kSumWords];
+	__shared__ double gam, rr, beta, dsub, alpha, delta, two[2], goal;
+	__shared__ int itrMax, stop, broke, iters, gaveUp, slow, sE[32], sFrame[2];
+	__shared__ unsigned tmemBase;
+	extern __shared__ __align__(128) char sdyn[];
+	CgScal *sc = a.sc;
+	if (sc->done) return;
+	constexpr int S = limb_stride<B>(), U = fix_u_stride<B>(), BB = B * B;
+	constexpr int kSlot = 256 * BB, kRing = many_slot<B>();
+	const int nctas = gridDim.x, lc = blockIdx.x, pw = a.pw;
+	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, W = blockDim.x >> 5;
+	const bool reducer = wp == W - 1, rowWarp = wp < pw;
+	const int oBar = pw * a.stages * kRing, oLimb = oBar + 8 * pw * a.stages, oHalo = oLimb + 8 * a.haloMax * S;
+	const int tslots = tmem_slots<B>(pw), oCol = (oHalo + 4 * a.haloMax + 15) & ~15;
+	int *slimb = (int *) (sdyn + oLimb), *shalo = (int *) (sdyn + oHalo);
+	unsigned short *tcol = (unsigned short *) (sdyn + oCol) + wp * tslots * 32 + lane;
+	char *ring = sdyn + wp * a.stages * kRing;
+	const unsigned mb = smem_addr(sdyn + oBar + 8 * wp * a.stages);
+	const int sl0 = lc * per * pw + wp;          // the warp's slice of chunk j: sl0 + j pw
+	const long vs = (long) nctas * per * pw * 32 * B;
+	for (int t = threadIdx.x, n = __ldg(a.haloNum + lc * per); t < n; t += blockDim.x)
+		shalo[t] = __ldg(a.halo + (long) lc * per * a.haloCap + t);
+	if (threadIdx.x == 0) {
+		gam = sc->gam; rr = sc->rr; beta = 0.0; dsub = 0.0; alpha = 1.0; delta = 0.0;
+		goal = sc->tolSqu * sc->bb; itrMax = sc->itrMax;
+		stop = -1; broke = -1; iters = 0; gaveUp = 0; slow = 0;
+	}
+	if (wp == 0) {
+		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_addr(&tmemBase)), "r"(kTmemCols) : "memory");
+		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+	}
+	__syncthreads();
+	const unsigned tmem = tmemBase + ((unsigned) (wp & 3) << 21) + (unsigned) ((wp >> 2) * tslots * 2 * BB);
+	auto slice_width = [&](int j) { return __ldg(a.width + sl0 + j * pw); };
+	// slots of chunk j that go through the ring; the others of chunk 0 stay in tensor memory
+	const int ntm = rowWarp ? min(tslots, slice_width(0)) : 0;
+	auto ring_slots = [&](int j) { return slice_width(j) - (j == 0 ? ntm : 0); };
+	if (ntm > 0) {
+		const int w0 = ring_slots(0), o = __ldg(a.off + sl0);
+		for (int k = 0; k < ntm; ++k) {
+			const int2 *g = (const int2 *) ((const char *) a.fix + (size_t) o * (8 * BB) + (size_t) (w0 + k) * kSlot) + lane;
+			int2 e[BB];
+#pragma unroll
+			for (int c = 0; c < B; ++c)
+#pragma unroll
+				for (int r = 0; r < B; ++r) e[c * B + r] = __ldg(g + (r * B + c) * 32);
+			tmem_store<B>(tmem + 2 * BB * k, e);
+			tcol[32 * k] = __ldg(a.lcol + o + (w0 + k) * 32 + lane);
+		}
+	}
+	int total = 0;                               // slots through the ring per matvec
+	if (rowWarp)
+		for (int j = 0; j < per; ++j) total += ring_slots(j);
+	const int nstage = min(a.stages, total);
+	unsigned long long policy;                   // the operator passes through L2, which keeps u and the rows' vectors
+	asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+	int nj = 0, nleft = 0;                       // chunk of the next load, and its slots not asked for yet
+	const char *nsrc = nullptr;                  // their entries and columns
+	const unsigned short *ncol = nullptr;
+	auto open_chunk = [&]() {
+		nleft = ring_slots(nj);
+		const int o = __ldg(a.off + sl0 + nj * pw);
+		nsrc = (const char *) a.fix + (size_t) o * (8 * BB);
+		ncol = a.lcol + o;
+	};
+	auto load_next = [&](int st) {               // every lane keeps the place, lane 0 issues
+		while (nleft == 0) { if (++nj == per) nj = 0; open_chunk(); }
+		if (lane == 0) {
+			const unsigned bar = mb + 8 * st;
+			asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"((unsigned) kRing) : "memory");
+			bulk_load_hint(ring + st * kRing, nsrc, kSlot, bar, policy);
+			bulk_load_hint(ring + st * kRing + kSlot, ncol, 64, bar, policy);
+		}
+		nsrc += kSlot;
+		ncol += 32;
+		--nleft;
+	};
+	if (rowWarp) {
+		if (lane == 0) {
+			for (int k = 0; k < nstage; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(mb + 8 * k) : "memory");
+			asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+			asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+		}
+		__syncwarp();
+		open_chunk();
+		for (int k = 0; k < nstage; ++k) load_next(k);
+		for (int j = 0; j < per; ++j) {
+			const int row = (sl0 + j * pw) * 32 + lane, i = __ldg(a.perm + row);
+			double *g = a.vec + (long) (sl0 + j * pw) * 32 * B + lane;
+#pragma unroll
+			for (int c = 0; c < B; ++c) {
+				const long k = (long) i * B + c;
+				g[32 * c] = i >= 0 ? a.x[k] : 0.0;
+				g[vs + 32 * c] = g[2 * vs + 32 * c] = 0.0;
+				g[3 * vs + 32 * c] = i >= 0 ? a.r0[k] : 0.0;
+			}
+		}
+	}
+	// stage(): halo values of a chunk into its buffer and the largest exponent; convert(): to digits in the frame e
+	auto stage_halo = [&](const int *rows, int nh, int *buf, int t0, int nt) {
+		int e = 1;
+#pragma unroll 4
+		for (int h = t0; h < nh; h += nt) {
+			double v[B];
+			load_halo<B>(a.ug + (long) rows[h] * U, v);
+			double *d = reinterpret_cast<double *>(buf + h * S);
+#pragma unroll
+			for (int c = 0; c < B; ++c) { d[c] = v[c]; e = max(e, fx_exp(v[c])); }
+		}
+		e = fx_warp_max(e);
+		if (lane == 0) sE[wp] = e;
+	};
+	auto convert_halo = [&](int nh, int *buf, int e, int t0, int nt) {
+#pragma unroll 1
+		for (int h = t0; h < nh; h += nt) {
+			double *d = reinterpret_cast<double *>(buf + h * S);
+#pragma unroll
+			for (int c = 0; c < B; ++c) {
+				int2 t;
+				limb_vector(d[c], e, t.x, t.y);
+				reinterpret_cast<int2 *>(d)[c] = t;
+			}
+		}
+	};
+	const int nstagers = W - 1 - pw;             // warps pw .. W - 2
+	int stage = 0;
+	unsigned parity = 0;
+	unsigned target = 0;
+	bool pending = false, first = true;
+	int line = 0;
+	__syncthreads();
+	for (;;) {
+		// (0) the first chunk's halo, by every warp but the reducer, which has the iteration's scalars to finish
+		const int nh0 = __ldg(a.haloNum + lc * per);
+		if (!reducer) stage_halo(shalo, nh0, slimb, threadIdx.x, 32 * (W - 1));
+		else if (pending) {
+			// lanes 0 and 1 share one division: g / gamma and g / alpha
+			const double g = two[0], q = two[1];
+			const double ratio = g / (lane == 1 ? alpha : gam);
+			const double ga = __shfl_sync(0xffffffffu, ratio, 1);
+			if (lane == 0) {
+				beta = ratio;
+				dsub = ratio * ga;
+				gam = g;
+				rr = q;
+				const int n = ++iters;
+				if (fx_exp(g) >= 2047 || fx_exp(q) >= 2047) stop = SA_ERR_NONFINITE;
+				else if (q < goal) stop = SA_OK;
+				else if (n >= itrMax) stop = SA_ERR_NOT_CONVERGED;
+			}
+		}
+		__syncthreads();
+		if (stop >= 0) break;
+		{
+			const int e = fx_warp_max(lane < W - 1 ? sE[lane] : 1);
+			if (threadIdx.x == 0) sFrame[0] = e;
+			if (!reducer) convert_halo(nh0, slimb, e, threadIdx.x, 32 * (W - 1));
+		}
+		__syncthreads();
+		// (1) chunk by chunk: w = A u, (w, u), p and s
+		double d1 = 0.0;
+		for (int j = 0; j < per; ++j) {
+			if (rowWarp) {
+				const int sl = sl0 + j * pw, row = sl * 32 + lane, nr = ring_slots(j), nt = j == 0 ? ntm : 0;
+				const int *uh = slimb + (j & 1) * a.haloMax * S;
+				const bool own = __ldg(a.perm + row) >= 0;
+				const int eRow = __ldg(a.rowExp + row);
+				double *g = a.vec + vs + (long) sl * 32 * B + lane;
+				double uv[B], pv[B], sv[B];
+				load_halo<B>(a.ug + (long) row * U, uv);
+#pragma unroll
+				for (int c = 0; c < B; ++c) { pv[c] = g[32 * c]; sv[c] = g[vs + 32 * c]; }
+				LimbSum acc[B];
+#pragma unroll
+				for (int c = 0; c < B; ++c) acc[c] = limb_zero();
+				int kt = 0;
+				for (int k = 0; k < nr; ++k) {
+					if (!ring_wait(mb + 8 * stage, parity)) gaveUp = 1;
+					const char *slot = ring + stage * kRing;
+					const int *u = uh + reinterpret_cast<const unsigned short *>(slot + kSlot)[lane] * S;
+					fix_slot_mac<B>(acc, reinterpret_cast<const int2 *>(slot) + lane, u);
+					__syncwarp();                // every lane has read the slot before it is overwritten
+					load_next(stage);
+					if (++stage == nstage) { stage = 0; parity ^= 1u; }
+					if (kt < nt && (kt + 1) * nr <= (k + 1) * nt) {
+						int2 t[BB];
+						tmem_load<B>(tmem + 2 * BB * kt, t);
+						tmem_slot_mac<B>(acc, t, uh + tcol[kt << 5] * S);
+						++kt;
+					}
+				}
+				for (; kt < nt; ++kt) {
+					int2 t[BB];
+					tmem_load<B>(tmem + 2 * BB * kt, t);
+					tmem_slot_mac<B>(acc, t, uh + tcol[kt << 5] * S);
+				}
+				if (own) {
+					const int eU = sFrame[j & 1];
+					const double be = beta;
+#pragma unroll
+					for (int c = 0; c < B; ++c) {
+						const double w = limb_to_double(acc[c], eRow, eU);
+						d1 += w * uv[c];
+						g[32 * c] = uv[c] + be * pv[c];
+						g[vs + 32 * c] = w + be * sv[c];
+					}
+				}
+			} else if (!reducer && j + 1 < per) {
+				const int ch = lc * per + j + 1, nh = __ldg(a.haloNum + ch), t0 = threadIdx.x - 32 * pw;
+				int *buf = slimb + ((j + 1) & 1) * a.haloMax * S;
+				stage_halo(a.halo + (long) ch * a.haloCap, nh, buf, t0, 32 * nstagers);
+				asm volatile("bar.sync 1, %0;" :: "r"(32 * nstagers) : "memory");
+				const int e = fx_warp_max(lane < nstagers ? sE[pw + lane] : 1);
+				if (t0 == 0) sFrame[(j + 1) & 1] = e;
+				convert_halo(nh, buf, e, t0, 32 * nstagers);
+			}
+			if (j + 1 < per) __syncthreads();    // the next chunk's digits are there, this one's have been read
+		}
+		const int fD[1] = {sum_frame(delta)};
+		{
+			const double t[1] = {d1};
+			if (!first) warp_digits<1>(t, fD, dig[wp]);
+		}
+		__syncthreads();
+		// (2) reducer: the grid's (w, u) and alpha
+		if (reducer && !first) {
+			double t[1];
+			bool flag = false;
+			const bool ok = sum_exchange<1>(dig[0], W, &a.gs->delta[line], nctas, fD, &a.gs->bar, t, flag);
+			if (lc == 0 && lane < kSumWords) a.gs->delta[line >= 1 ? line - 1 : 2].w[lane] = 0ull;
+			if (lane == 0) {
+				if (!ok) gaveUp = 1;
+				slow = flag ? 1 : 0;
+				if (!flag) {
+					delta = t[0];
+					alpha = gam / (t[0] - dsub);
+					// bits, not FP64 compares (64 clocks each): alpha positive and finite, beta finite
+					if (__double_as_longlong(alpha) <= 0 || fx_exp(alpha) >= 2047 || fx_exp(beta) >= 2047)
+						broke = fx_exp(t[0]) < 2047 ? SA_ERR_BREAKDOWN : SA_ERR_NONFINITE;
+				}
+			}
+		}
+		__syncthreads();
+		if (first || slow) {
+			if (!gaveUp && !slow_sum<1>(d1, 0.0, two, a.part, nctas, &a.gs->bar, target, fs)) {
+				if (threadIdx.x == 0) gaveUp = 1;
+			} else if (threadIdx.x == 0 && !gaveUp) {
+				delta = two[0];
+				alpha = gam / (delta - dsub);
+				if (!(alpha > 0.0) || !isfinite(alpha) || !isfinite(beta))
+					broke = isfinite(delta) ? SA_ERR_BREAKDOWN : SA_ERR_NONFINITE;
+			}
+			__syncthreads();
+		}
+		if (gaveUp || broke >= 0) break;
+		const double al = alpha;
+		// (3) rows: r, u and (r, u), (r, r); the reducer adds them over the grid, which also completes u
+		double d2[2] = {0.0, 0.0};
+		if (rowWarp)
+#pragma unroll 1
+			for (int j = 0; j < per; ++j) {
+				const int sl = sl0 + j * pw;
+				double *g = a.vec + 2 * vs + (long) sl * 32 * B + lane;
+				const double *mi = a.pinv + (long) sl * 32 * BB + lane;
+				double rv[B], sv[B], uv[B], m[BB];
+#pragma unroll
+				for (int c = 0; c < B; ++c) { rv[c] = g[vs + 32 * c]; sv[c] = g[32 * c]; }
+#pragma unroll
+				for (int t = 0; t < BB; ++t) m[t] = __ldg(mi + 32 * t);
+#pragma unroll
+				for (int c = 0; c < B; ++c) { rv[c] = rv[c] - al * sv[c]; g[vs + 32 * c] = rv[c]; }
+#pragma unroll
+				for (int r = 0; r < B; ++r) {
+					double t = m[r * B] * rv[0];
+#pragma unroll
+					for (int c = 1; c < B; ++c) t += m[r * B + c] * rv[c];
+					uv[r] = t;
+				}
+				double2 *o = reinterpret_cast<double2 *>(a.ug + (long) (sl * 32 + lane) * U);
+				o[0] = make_double2(uv[0], uv[1]);
+				if constexpr (B == 3) o[1] = make_double2(uv[2], 0.0);
+#pragma unroll
+				for (int c = 0; c < B; ++c) { d2[0] += rv[c] * uv[c]; d2[1] += rv[c] * rv[c]; }
+			}
+		const int fG[2] = {sum_frame(gam), sum_frame(rr)};
+		warp_digits<2>(d2, fG, dig[wp]);
+		__syncthreads();
+		if (reducer) {
+			double t[2];
+			bool flag = false;
+			__threadfence();                     // the CTA's u before its count
+			const bool ok = sum_exchange<2>(dig[0], W, &a.gs->gamma[line], nctas, fG, &a.gs->bar, t, flag);
+			if (lc == 0 && lane < kSumWords) a.gs->gamma[line >= 1 ? line - 1 : 2].w[lane] = 0ull;
+			if (lane == 0) {
+				if (!ok) gaveUp = 1;
+				slow = flag ? 1 : 0;
+				two[0] = t[0];
+				two[1] = t[1];
+			}
+		} else if (rowWarp) {
+#pragma unroll 1
+			for (int j = 0; j < per; ++j) {      // while the reducer waits
+				double *g = a.vec + (long) (sl0 + j * pw) * 32 * B + lane;
+				double xv[B], pv[B];
+#pragma unroll
+				for (int c = 0; c < B; ++c) { xv[c] = g[32 * c]; pv[c] = g[vs + 32 * c]; }
+#pragma unroll
+				for (int c = 0; c < B; ++c) g[32 * c] = xv[c] + al * pv[c];
+			}
+		}
+		__syncthreads();
+		if (gaveUp) break;
+		if (slow) {
+			if (!slow_sum<2>(d2[0], d2[1], two, a.part + nctas, nctas, &a.gs->bar, target, fs)) {
+				if (threadIdx.x == 0) gaveUp = 1;
+				__syncthreads();
+				break;
+			}
+		}
+		if (++line == 3) line = 0;
+		pending = true;
+		first = false;
+	}
+	if (rowWarp) {
+		for (int j = 0; j < per; ++j) {
+			const int i = __ldg(a.perm + (sl0 + j * pw) * 32 + lane);
+			const double *g = a.vec + (long) (sl0 + j * pw) * 32 * B + lane;
+			if (i >= 0)
+#pragma unroll
+				for (int c = 0; c < B; ++c) a.x[(long) i * B + c] = g[32 * c];
+		}
+		for (int k = 0; k < nstage; ++k) {       // the ring's copies in flight land before the CTA leaves
+			ring_wait(mb + 8 * stage, parity);
+			if (++stage == nstage) { stage = 0; parity ^= 1u; }
+		}
+	}
+	__syncthreads();
+	if (wp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmemBase), "r"(kTmemCols));
+	if (lc == 0 && threadIdx.x == 0) {
+		sc->iters = iters; sc->code = gaveUp ? SA_ERR_TIMEOUT : max(stop, broke); sc->rr = rr; sc->gam = gam; sc->done = 1;
+	}
+}
+
 template <int B>
 bool cgfix_run(const Mesh &m, const double *blk, const double *binv, double *x, const double *r, const double *u,
                CgWork &w, cudaEvent_t e0, cudaEvent_t e1, cudaStream_t s)
@@ -741,44 +1143,59 @@ bool cgfix_run(const Mesh &m, const double *blk, const double *binv, double *x, 
 	const CgPlan &p = w.plan;
 	if (!p.ok || m.dim != B) return false;
 	static std::mutex mu;
-	static size_t limits[2];
+	static size_t limits[3];
 	static bool known = false;
 	{
 		std::lock_guard<std::mutex> g(mu);
 		if (!known) {
 			limits[0] = fix_smem_limit((const void *) k_cg_fix<B, false>);
 			limits[1] = fix_smem_limit((const void *) k_cg_fix<B, true>);
+			limits[2] = fix_smem_limit((const void *) k_cg_fix_many<B>);
 			known = true;
 		}
 	}
-	const size_t lim = std::min(limits[0], limits[1]);
 	const int colMax = 32 * p.pw * p.widest;
 	const size_t perStage = (size_t) p.pw * (256 * B * B + 8);
-	const bool resident = fix_smem<B>(p.pw, p.parts, p.haloMax, colMax, p.widest) <= lim;
-	const int parts = resident ? p.parts : 1;
-	const size_t fixed = fix_smem<B>(p.pw, parts, p.haloMax, colMax, 0);
-	if (p.nchunk > kSumMaxCtas || (!resident && fixed + 2 * perStage > lim)) return false;
-	const int stages = resident ? p.widest : (int) ((lim - fixed) / perStage);
-	const size_t smem = fix_smem<B>(p.pw, parts, p.haloMax, colMax, stages);
-	const void *kernel = resident ? (const void *) k_cg_fix<B, false> : (const void *) k_cg_fix<B, true>;
+	int parts = 1, stages, per = p.per;
+	size_t smem;
+	const void *kernel;
+	if (per > 1) {
+		const size_t lim = limits[2], fixed = fix_many_smem<B>(p.pw, p.haloMax, 0);
+		const size_t perStage = (size_t) p.pw * (many_slot<B>() + 8);
+		if (fixed + 2 * perStage > lim) return false;
+		stages = (int) ((lim - fixed) / perStage);
+		smem = fix_many_smem<B>(p.pw, p.haloMax, stages);
+		kernel = (const void *) k_cg_fix_many<B>;
+	} else {
+		const size_t lim = std::min(limits[0], limits[1]);
+		const bool resident = fix_smem<B>(p.pw, p.parts, p.haloMax, colMax, p.widest) <= lim;
+		parts = resident ? p.parts : 1;
+		const size_t fixed = fix_smem<B>(p.pw, parts, p.haloMax, colMax, 0);
+		if (!resident && fixed + 2 * perStage > lim) return false;
+		stages = resident ? p.widest : (int) ((lim - fixed) / perStage);
+		smem = fix_smem<B>(p.pw, parts, p.haloMax, colMax, stages);
+		kernel = resident ? (const void *) k_cg_fix<B, false> : (const void *) k_cg_fix<B, true>;
+	}
+	const int nctas = p.nchunk / per;
 	int occ = 0;
 	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 32 * p.warps, smem) != cudaSuccess) {
 		cudaGetLastError();
 		return false;
 	}
-	if (p.nchunk > occ * w.smCount) return false;
+	if (nctas > occ * w.smCount || nctas > kSumMaxCtas) return false;
 	const int P = p.nchunk * 32 * p.pw;
 	k_cgfix_operator<B><<<(p.nslice + 3) / 4, 128, 0, s>>>(p.nslice, sell_of(m), m.rowPtr, blk, p.perm, p.width, p.off,
 	                                                       p.fix, p.rowExp);
 	k_cgfix_gather_copy<B><<<grid_for(P), kBlock, 0, s>>>(P, p.perm, u, p.ug);
+	if (per > 1) k_cgfix_inverses<B><<<grid_for(P), kBlock, 0, s>>>(P, p.perm, binv, p.pinv);
 	SA_CHECK(cudaMemsetAsync(w.bar, 0, sizeof(GridSums), s));
 	FixArgs a{p.pw, parts, p.haloCap, p.haloMax, colMax, stages, p.perm, p.width, p.off, p.halo, p.haloNum, p.rowExp, p.lcol, p.fix,
-	          binv, r, u, x, p.ug, p.vec, w.part, (CgScal *) w.scal, (GridSums *) w.bar};
-	void *args[] = {&a};
+	          binv, r, u, x, p.ug, p.vec, w.part, p.pinv, (CgScal *) w.scal, (GridSums *) w.bar};
+	void *args[] = {&a, &per};
 	if (e0) SA_CHECK(cudaEventRecord(e0, s));
-	SA_CHECK(cudaLaunchCooperativeKernel(kernel, dim3(p.nchunk), dim3(32 * p.warps), args, smem, s));
+	SA_CHECK(cudaLaunchCooperativeKernel(kernel, dim3(nctas), dim3(32 * p.warps), args, smem, s));
 	if (e1) SA_CHECK(cudaEventRecord(e1, s));
-	w.launches += 3;
+	w.launches += per > 1 ? 4 : 3;
 	return true;
 }
 

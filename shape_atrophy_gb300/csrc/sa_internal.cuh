@@ -473,6 +473,7 @@ struct CgPlan {
 	bool ok = false;              // built, and every chunk's halo fits
 	int nchunk = 0, pw = 0, warps = 0, nslice = 0, widest = 0, haloCap = 0, haloMax = 0;
 	int parts = 1;                // warps that share a slice's slots (small chunks)
+	int per = 1;                  // chunks per CTA (large operators)
 	long total = 0;               // slots of the permuted sliced layout
 	int *perm = nullptr;          // nchunk 32 pw: node of each permuted row (-1: padding)
 	int *inv = nullptr;           // N: permuted row of each node
@@ -483,6 +484,7 @@ struct CgPlan {
 	int *rowExp = nullptr;        // nchunk 32 pw: largest exponent field of each permuted row
 	double *ug = nullptr;         // the gather copy of u in permuted order (3-component nodes padded to 4)
 	double *vec = nullptr;        // x, p, s and r of the permuted rows, [vector][slice][component][lane]
+	double *pinv = nullptr;       // block inverses in that order (several chunks per CTA)
 };
 
 struct CgWork {            // scratch of the Jacobi CG (Chronopoulos-Gear form)

@@ -3,7 +3,8 @@
 Both solve the same systems to the relative residual 1e-12, so a step's velocities differ by that times the operator's
 condition; the bound, 1e-10 relative in positions and concentration, is the one the solver paths are held to against
 the oracle.  Sizes: fewer rows than a warp, one row more than a slice, several warps per slice, one warp per slice,
-slices that outgrow shared memory (tensor memory and streamed slots), and rows wide enough to be refused (FP64 kernels).
+slices that outgrow shared memory (tensor memory and streamed slots), several chunks per CTA (108 027 rows in 2-D, 122 886
+in 3-D), and rows wide enough to be refused (FP64 kernels).
 """
 import numpy as np
 import pytest
@@ -26,7 +27,8 @@ def _spec(kind, a, b):
 
 @pytest.mark.parametrize("kind,a,b", [("annulus", 5, 4), ("annulus", 11, 3), ("annulus", 97, 13), ("annulus", 610, 8),
                                       ("annulus", 1201, 17), ("shell", 0, 2), ("shell", 1, 3), ("shell", 2, 4),
-                                      ("shell", 3, 9), ("shell", 4, 5), ("shell", 4, 9), ("shell", 5, 6)])
+                                      ("shell", 3, 9), ("shell", 4, 5), ("shell", 4, 9), ("shell", 5, 6),
+                                      ("annulus", 4001, 27), ("shell", 6, 3)])
 def test_matches_two_kernel_cg(kind, a, b):
     from shape_atrophy_gb300 import api
     spec = _spec(kind, a, b)

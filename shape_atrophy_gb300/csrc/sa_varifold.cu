@@ -10,7 +10,9 @@
 //   dsum (2D_frame/dsum.cu:6-73)                     -> device_sum (same 512-wide tree order)
 // The Matern-3/2 centre kernel 'M' (1 + r/w) exp(-r/w) is the layered model's addition.
 //
-// FP64 pair term: e^x by a table-driven method and the Matern distance by a
+// FP64 objective with the kernels 'M', 'G' and 'B', 'L': pair terms in fixed point (k_vfd_rows_fix).
+//
+// FP64 pair term elsewhere: e^x by a table-driven method and the Matern distance by a
 // Newton square root (exp_tab, sqrt_nr below), both within about 1 ulp;
 // work items (row block, column chunk) taken largest first by a persistent
 // grid.
@@ -24,6 +26,7 @@
 // evaluated again in FP64, with both element sets in Morton order so that a
 // warp's rows take that branch together (spatial_order).
 #include "sa_internal.cuh"
+#include "sa_pairfix.cuh"
 #include <cmath>
 #include <algorithm>
 
@@ -449,6 +452,132 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 }
 
 // ---------------------------------------------------------------------------
+// The same row sums, without gradient, with the pair terms in fixed point (sa_pairfix.cuh): centre kernels 'M' and 'G',
+// direction kernels 'B' and 'L'.  A tile's directions and volumes are digits in the frame of its largest, its terms
+// are added in integers, and the sum is rounded to FP64 once per tile.
+//
+// Two sets of 20 480 triangles, 'M' x 'B' (840 million pairs): 53.5 ms with the FP64 pair terms of k_vfd_rows (30 FP64 operations
+// a pair), 12.1 ms here; 580 clocks per pair and warp, of which the six FP64 operations of the squared distance take 384
+// and the rest is integer issue.  The other kernels ('C' needs a reciprocal, 'O' and 'U' a second exponential of either
+// sign) and gradient rows stay in FP64, as does the path without allocation.  Against 128-bit sums, 24 curves of 100 to
+// 1000 segments: root mean square error 2.1e-16 of the self term, FP64 pair terms 2.2e-16.
+// ---------------------------------------------------------------------------
+__constant__ unsigned long long c_pair_exp[256] = {SA_PAIR_EXP_TABLE};
+
+struct __align__(16) PairColumn {
+	double2 c01;                              // centre in widths
+	double c2;
+	unsigned long long v;                     // volume at 63 bits, bit 63 its sign
+	int4 q0;                                  // direction digits: high 0, 1, 2, low 0
+	int2 q1;                                  // low 1, 2
+	int2 pad;
+};
+
+template <int D, int CK>
+__global__ void __launch_bounds__(kVfdTile) k_vfd_rows_fix(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, double cw, int dk,
+                                                           double *__restrict__ out, int symA, int C, int *__restrict__ queue)
+{
+	__shared__ PairColumn col[kVfdTile];
+	__shared__ unsigned long long tab[256];
+	__shared__ int sItem, sU[kVfdTile / 32], sV[kVfdTile / 32];
+	const double cs = 1.0 / cw;
+	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+	for (int t = threadIdx.x; t < 256; t += kVfdTile) tab[t] = c_pair_exp[t];
+	const int rowBlocks = (R.n + kVfdTile - 1) / kVfdTile, nItems = rowBlocks * C;
+	for (;;) {
+		__syncthreads();                      // the previous item's reads are done
+		if (threadIdx.x == 0) sItem = atomicAdd(queue, 1);
+		__syncthreads();
+		const int item = sItem;
+		if (item >= nItems) break;
+		const int bx = item / C, cy = item % C, i = bx * kVfdTile + threadIdx.x;
+		const bool act = i < R.n;
+		double ci[D], ui[D], n2 = 0.0, acc = 0.0;
+		bool bad = false;                     // a value that is not finite: the sums are NaN
+		for (int d = 0; d < D; ++d) {
+			ci[d] = act ? R.cen[d * (long) R.n + i] * cs : 0.0;
+			ui[d] = act ? R.dir[d * (long) R.n + i] : 0.0;
+			n2 = fma(ui[d], ui[d], n2);
+			bad = bad || fx_exp(ci[d]) >= 2047;
+		}
+		const int eRow = pair_frame(n2);
+		bad = bad || fx_exp(n2) >= 2047;
+		int uh[D], ul[D];
+		for (int d = 0; d < D; ++d) pair_digits(bad ? 0.0 : scalbn(ui[d], -eRow), uh[d], ul[d]);
+		for (int set = 0; set < 2; ++set) {
+			const VfdSet &S = set == 0 ? A : Bs;
+			const double cv = (set == 0 ? cA : cB) * (act ? R.vol[i] : 0.0);
+			const bool sym = set == 0 && symA;
+			const int lo = sym ? bx * kVfdTile : 0;                 // columns below the item's rows: none
+			const int span = S.n > lo ? S.n - lo : 0;
+			const int jBeg = lo + (int) ((long) span * cy / C), jEnd = lo + (int) ((long) span * (cy + 1) / C);
+			for (int j0 = jBeg; j0 < jEnd; j0 += kVfdTile) {
+				const int nt = min(kVfdTile, jEnd - j0), t = threadIdx.x;
+				double c[3] = {0.0, 0.0, 0.0}, u[3] = {0.0, 0.0, 0.0}, v = 0.0, m2 = 0.0;
+				int e = 0;
+				if (t < nt) {
+					for (int d = 0; d < D; ++d) {
+						c[d] = S.cen[d * (long) S.n + j0 + t] * cs;
+						u[d] = S.dir[d * (long) S.n + j0 + t];
+						m2 = fma(u[d], u[d], m2);
+						e = max(e, fx_exp(c[d]));
+					}
+					v = S.vol[j0 + t];
+				}
+				const int eu = __reduce_max_sync(0xffffffffu, fx_exp(m2) >= 2047 ? 1024 : pair_frame(m2));
+				const int ev = __reduce_max_sync(0xffffffffu, e >= 2047 ? 2047 : fx_exp(v));
+				if (lane == 0) { sU[wp] = eu; sV[wp] = ev; }
+				__syncthreads();              // the frames; the previous tile has been read
+				int eU = sU[0], eV = sV[0];
+				for (int w = 1; w < kVfdTile / 32; ++w) { eU = max(eU, sU[w]); eV = max(eV, sV[w]); }
+				const bool tileBad = eU >= 1024 || eV >= 2047;
+				eV -= 1022;                   // |v| < 2^eV
+				if (!tileBad) {
+					int h[3] = {0, 0, 0}, l[3] = {0, 0, 0};
+					for (int d = 0; d < D; ++d) pair_digits(scalbn(u[d], -eU), h[d], l[d]);
+					col[t].c01 = make_double2(c[0], c[1]);
+					col[t].c2 = c[2];
+					col[t].v = (unsigned long long) __double2ll_rn(scalbn(fabs(v), 63 - eV)) |
+					           (__double2hiint(v) < 0 ? 1ull << 63 : 0ull);
+					col[t].q0 = make_int4(h[0], h[1], h[2], l[0]);
+					col[t].q1 = make_int2(l[1], l[2]);
+				}
+				__syncthreads();
+				if (act && (tileBad || bad)) acc = __longlong_as_double(0x7ff8000000000000ll);
+				if (act && !tileBad && !bad) {
+					// sum of the terms as hi 2^32 + lo: 128 terms below 2^61
+					long long hi = 0, dg = 0;
+					unsigned long long lo32 = 0;
+					for (int jj = sym ? max(0, i - j0) : 0; jj < nt; ++jj) {
+						const double2 c01 = col[jj].c01;
+						const double dx = ci[0] - c01.x, dy = ci[1] - c01.y;
+						double d2 = dx * dx + dy * dy;
+						if constexpr (D == 3) { const double dz = ci[2] - col[jj].c2; d2 = d2 + dz * dz; }
+						const int4 q0 = col[jj].q0;
+						const int2 q1 = col[jj].q1;
+						const int vh[3] = {q0.x, q0.y, q0.z}, vl[3] = {q0.w, q1.x, q1.y};
+						bool neg;
+						int m;
+						const unsigned long long ang = pair_angle<D>(uh, ul, vh, vl, neg);
+						const unsigned long long kc = pair_centre(CK, (unsigned) __double2hiint(d2), (unsigned) __double2loint(d2), m, tab);
+						const unsigned long long w = col[jj].v;
+						long long s = (long long) pair_term(kc, m, dk, ang, w & ~(1ull << 63));
+						if ((neg && dk == 'L') != ((long long) w < 0)) s = -s;
+						hi += s >> 32;
+						lo32 += (unsigned) s;
+						if (sym && j0 + jj == i) dg = s;
+					}
+					double ts = fma((double) hi, 0x1p32, (double) lo32);
+					if (sym) ts = 2.0 * ts - (double) dg;
+					acc += cv * scalbn(ts, (dk == 'B' ? 2 : 1) * (eRow + eU) + eV - 61);
+				}
+			}
+		}
+		if (act) out[(long) cy * R.n + i] = acc;
+	}
+}
+
+// ---------------------------------------------------------------------------
 // Spatial order of a set of boundary elements (mixed-precision objective).
 // The FP64 near-field branch of the FP32 pair sums is taken by a warp when
 // any of its 32 rows is near the column; in mesh order a warp's rows lie all
@@ -704,29 +833,34 @@ double device_sum(const double *v, long n, double *scratch, cudaStream_t s)
 	return h;
 }
 
-constexpr int kVfdBlock = 128;
+constexpr int kVfdBlock = kVfdTile;
 
-// persistent grid of k_vfd_rows: as many CTAs as fit on the GPU at once, at most one per work item
-template <int D, typename T, bool G>
-static int vfd_grid(int items)
+// persistent grid of a pair-sum kernel: as many CTAs as fit on the GPU at once, at most one per work item
+static int vfd_grid(const void *kernel, int items)
 {
 	int dev = 0, sms = 1, per = 1;
 	SA_CHECK(cudaGetDevice(&dev));
 	SA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-	SA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_vfd_rows<D, T, G>, kVfdBlock, 0));
+	SA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kVfdBlock, 0));
 	return std::max(1, std::min(items, std::max(1, per) * sms));
 }
 
-// one k_vfd_rows launch over all (row block, column chunk) items of R, taken from the queue counter (zeroed
-// here on the stream)
+// one launch over all (row block, column chunk) items of R, taken from the queue counter (zeroed here on the stream)
 template <int D, typename T, bool G>
 static void launch_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet B, double cB, int ck, double cw, int dk, double dw,
                             double *out, double *dc, double *dt, int sym, int C, int *queue, cudaStream_t s)
 {
 	const int items = grid_for(R.n, kVfdBlock) * C;
 	SA_CHECK(cudaMemsetAsync(queue, 0, sizeof(int), s));
-	k_vfd_rows<D, T, G><<<vfd_grid<D, T, G>(items), kVfdBlock, 0, s>>>(R, A, cA, B, cB, ck, cw, dk, dw, out, dc, dt,
-	                                                                     sym, C, queue);
+	if constexpr (!G && sizeof(T) == sizeof(double)) {
+		if ((ck == 'M' || ck == 'G') && (dk == 'B' || dk == 'L')) {
+			auto kernel = ck == 'M' ? k_vfd_rows_fix<D, 'M'> : k_vfd_rows_fix<D, 'G'>;
+			kernel<<<vfd_grid((const void *) kernel, items), kVfdBlock, 0, s>>>(R, A, cA, B, cB, cw, dk, out, sym, C, queue);
+			return;
+		}
+	}
+	k_vfd_rows<D, T, G><<<vfd_grid((const void *) k_vfd_rows<D, T, G>, items), kVfdBlock, 0, s>>>(
+		R, A, cA, B, cB, ck, cw, dk, dw, out, dc, dt, sym, C, queue);
 }
 
 // column chunks of the pair sums of a Vd x Vt objective: enough CTAs to fill the GPU (the pair sums are latency

@@ -618,7 +618,7 @@ template <int D> double varifold(const Mesh &m, const Model &md, const double *x
                                  cudaStream_t s, int precision, int *err, VfdTargetCache *cache = nullptr);
 
 // column chunks of the varifold pair sums of a Vd x Vt objective
-int vfd_chunk_count(int Vd, int Vt);
+int vfd_chunk_count(int Vd, int Vt, int precision);
 // the target-target rows of a Vd x Vt objective into cache.rows on stream s (the objective's own launches);
 // part: varifold_target_rows_scratch(D, Vd, Vt, precision) doubles
 size_t varifold_target_rows_scratch(int D, int Vd, int Vt, int precision);

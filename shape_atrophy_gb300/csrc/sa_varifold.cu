@@ -866,9 +866,10 @@ static void launch_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet B, double cB, 
 // column chunks of the pair sums of a Vd x Vt objective: enough CTAs to fill the GPU (the pair sums are latency
 // bound at one CTA per SM), each chunk at least kVfdMinCols columns wide.  A warp alone on its sub-partition issues an
 // FP64 operation every 64 clocks whatever the chunk, so small sets want many narrow chunks: 512 x 512 segments with
-// gradient, 256 columns per chunk 0.9 ms in the pair sums, 16 columns 0.1 ms.
+// gradient, 256 columns per chunk 0.9 ms in the pair sums, 16 columns 0.1 ms.  Mixed precision rounds at the ends of its
+// tiles of 128 columns (relative 1e-9 of the objective moves with them), so its chunks stay two tiles wide.
 constexpr int kVfdMinCols = 16;
-int vfd_chunk_count(int Vd, int Vt)
+int vfd_chunk_count(int Vd, int Vt, int precision)
 {
 	int dev = 0, sms = 1;
 	SA_CHECK(cudaGetDevice(&dev));
@@ -877,7 +878,7 @@ int vfd_chunk_count(int Vd, int Vt)
 	const int perSm = std::max(1, tuning().vfdCtasPerSm);
 	const int rowCtas = std::max(1, grid_for(rowMax, kVfdBlock));
 	int C = std::max(1, (perSm * sms + rowCtas - 1) / rowCtas);
-	C = std::min(C, std::max(1, colMin / kVfdMinCols));
+	C = std::min(C, std::max(1, colMin / (precision == SA_PREC_MIXED ? 2 * kVfdTile : kVfdMinCols)));
 	return std::min(C, 32);
 }
 
@@ -886,7 +887,7 @@ int vfd_chunk_count(int Vd, int Vt)
 // cache or computes them itself.  part: varifold_target_rows_scratch(D, Vd, Vt, precision) doubles.
 size_t varifold_target_rows_scratch(int D, int Vd, int Vt, int precision)
 {
-	return (size_t) vfd_chunk_count(Vd, Vt) * Vt + (precision == SA_PREC_MIXED ? spatial_order_doubles(D, Vt) : 0) +
+	return (size_t) vfd_chunk_count(Vd, Vt, precision) * Vt + (precision == SA_PREC_MIXED ? spatial_order_doubles(D, Vt) : 0) +
 	       1;                                                      // + the work-item counter
 }
 
@@ -895,7 +896,7 @@ void varifold_target_rows(const Model &md, int Vd, const double *tgtCen, const d
                           int Vt, int precision, double *part, VfdTargetCache &cache, cudaStream_t s)
 {
 	if (!cache.rows || cache.capacity < Vt || Vt <= 0) return;     // not cached: the objective computes them
-	const int C = vfd_chunk_count(Vd, Vt);
+	const int C = vfd_chunk_count(Vd, Vt, precision);
 	VfdSet Ts{tgtCen, tgtDir, tgtVol, Vt}, E0{nullptr, nullptr, nullptr, 0};
 	int *queue = reinterpret_cast<int *>(part + varifold_target_rows_scratch(D, Vd, Vt, precision) - 1);
 	if (precision == SA_PREC_MIXED) Ts = spatial_order<D>(Ts, part + (size_t) C * Vt, s);
@@ -925,7 +926,7 @@ double varifold(const Mesh &m, const Model &md, const double *x, const double *t
 	*err = SA_OK;
 	if (grad && !m.vfdIfo) { *err = SA_ERR_ARG; return 0.0; }
 	const int rowMax = std::max(Vd, Vt);
-	const int C = vfd_chunk_count(Vd, Vt);
+	const int C = vfd_chunk_count(Vd, Vt, precision);
 	double *buf = nullptr;
 	const size_t rows = (size_t) (Vd + Vt);
 	// mixed-precision objective: both sets in spatial order (coherent near-field branch, see spatial_order)

@@ -149,10 +149,58 @@ SA_FX_HD unsigned long long pair_sqrt(unsigned hi, unsigned lo)
 	return k == 6 ? s << 1 : s >> (5 - k);
 }
 
-// K_c at 63 + m bits: 'M' (1 + r) e^-r, 'G' e^-d2; d2 the squared distance in widths
+// 1 / a at 63 + m bits for a double a >= 1 (0 from 2^62 on): Y the FP32 reciprocal of the significand A in [1, 2), e = 1 - A Y,
+// 1 / A = Y (1 + e + e^2); |e| < 2^-21
+SA_FX_HD unsigned long long pair_recip(unsigned hi, unsigned lo, int &m)
+{
+	m = (int) (hi >> 20) - 1023;
+	if (m >= 62) return 0ull;
+	const unsigned top = (hi & 0xfffffu) | 0x100000u;
+	const unsigned long long A = (((unsigned long long) top << 32) | lo) << 10;                   // 62 bits
+	const unsigned bits = (127u << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+#ifdef __CUDA_ARCH__
+	float y;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(bits)));
+	const unsigned Y = __float2uint_rz(y * 536870912.0f) << 1;                                    // 30 bits, even
+#else
+	float f;
+	__builtin_memcpy(&f, &bits, 4);
+	const unsigned Y = (unsigned) (1.0f / f * 536870912.0f) << 1;
+#endif
+	const unsigned long long P = (((A >> 32) * Y) << 2) + (((A & 0xffffffffull) * Y) >> 30);      // A Y at 62 bits
+	const long long e = (long long) ((1ull << 62) - P);
+	const int eh = (int) (e >> 12);                                                               // 50 bits
+	const long long s = e + (((long long) eh * eh) >> 38);
+	const long long c = (((s >> 12) * (long long) (int) (Y >> 1)) >> 16) + (((s & 0xfff) * (long long) (int) (Y >> 1)) >> 28);
+	return ((unsigned long long) Y << 33) + c;
+}
+
+// v 2^-b as a double, v below 2^64; rounded once
+SA_FX_HD double pair_double(unsigned long long v, int b)
+{
+#ifdef __CUDA_ARCH__
+	const int n = __clzll((long long) v);
+#else
+	const int n = v ? __builtin_clzll(v) : 64;
+#endif
+	if (n == 64 || b > 1000) return 0.0;
+	const unsigned long long q = (v << n) >> 10;              // 54 bits
+	const unsigned long long r = ((unsigned long long) (1023 + 62 - n - b) << 52) + ((q + 1ull) >> 1);   // the leading bit adds one
+#ifdef __CUDA_ARCH__
+	return __longlong_as_double((long long) r);
+#else
+	double d;
+	__builtin_memcpy(&d, &r, 8);
+	return d;
+#endif
+}
+
+// K_c at 63 + m bits: 'M' (1 + r) e^-r, 'G' e^-d2, 'C' 1 / a; hi and lo the words of the squared distance d2 in widths ('C': of
+// a = 1 + d2)
 SA_FX_HD unsigned long long pair_centre(int type, unsigned hi, unsigned lo, int &m, const unsigned long long *tab)
 {
 	if (type == 'G') return pair_exp(pair_fix(hi, lo), m, tab);
+	if (type == 'C') return pair_recip(hi, lo, m);
 	const unsigned long long r = pair_sqrt(hi, lo), e = pair_exp(r, m, tab);
 	unsigned long long v = pair_mulh(r + (1ull << 57), e);   // 56 bits, below 2^m
 	if (m < 7) v <<= 7 - m;
@@ -182,10 +230,9 @@ SA_FX_HD unsigned long long pair_angle(const int *uh, const int *ul, const int *
 	return (unsigned long long) (neg ? -s : s) << 1;
 }
 
-// K_c K_d v at 61 bits; v at 63.  type: 'B' (u_i . u_j)^2, 'L' u_i . u_j (the sign is the caller's)
-SA_FX_HD unsigned long long pair_term(unsigned long long kc, int m, int type, unsigned long long ang, unsigned long long v)
+// K_c K_d v at 61 bits from K_c at 63 + m, K_d and v at 63
+SA_FX_HD unsigned long long pair_term(unsigned long long kc, int m, unsigned long long kd, unsigned long long v)
 {
-	const unsigned long long kd = type == 'B' ? pair_mulh(ang, ang) << 1 : ang;
 	const unsigned long long q = pair_mulh(kc, pair_mulh(kd, v));
 	m = m < 63 ? m : 63;
 	return (q + ((1ull << m) >> 1)) >> m;

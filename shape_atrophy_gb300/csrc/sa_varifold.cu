@@ -10,9 +10,9 @@
 //   dsum (2D_frame/dsum.cu:6-73)                     -> device_sum (same 512-wide tree order)
 // The Matern-3/2 centre kernel 'M' (1 + r/w) exp(-r/w) is the layered model's addition.
 //
-// FP64 objective with the kernels 'M', 'G' and 'B', 'L': pair terms in fixed point (k_vfd_rows_fix).
+// FP64 objective: pair terms in fixed point (k_vfd_rows_fix); FP64 gradient rows: kernel values in fixed point.
 //
-// FP64 pair term elsewhere: e^x by a table-driven method and the Matern distance by a
+// FP64 pair term elsewhere (the path without allocation, the mixed objective's near field): e^x by a table-driven method and the Matern distance by a
 // Newton square root (exp_tab, sqrt_nr below), both within about 1 ulp;
 // work items (row block, column chunk) taken largest first by a persistent
 // grid.
@@ -102,6 +102,8 @@ __constant__ double c_exp2_256[256] = {
 	0x1.f50765b6e4540p+0, 0x1.f6632798844f8p+0, 0x1.f7bfdad9cbe14p+0, 0x1.f91d802243c89p+0,
 	0x1.fa7c1819e90d8p+0, 0x1.fbdba3692d514p+0, 0x1.fd3c22b8f71f1p+0, 0x1.fe9d96b2a23d9p+0,
 };
+
+__constant__ unsigned long long c_pair_exp[256] = {SA_PAIR_EXP_TABLE};
 
 // e^x in FP64 by Tang's table-driven method (P. T. P. Tang, "Table-driven implementation of the
 // exponential function in IEEE floating-point arithmetic", ACM TOMS 15(2), 1989): with
@@ -198,17 +200,52 @@ __device__ __forceinline__ T dir_knl(int type, T iw2, T ang, T &d1, const double
 }
 
 // The gradient rows' FP64 work per pair is what bounds them (5120 x 5120 triangles, 'C' x 'O': 12.1 -> 7.2 ms a call when
-// the divisions, the width scalings and the row factors left the pair loop).
+// the divisions, the width scalings and the row factors left the pair loop, 4.3 ms when the kernel values were
+// formed in fixed point, sa_pairfix.cuh, and converted).
+// e^-x; outside [0, 64) by exp_tab
+__device__ __forceinline__ double exp_fix(double x, const unsigned long long *ptab, const double *tab)
+{
+	const unsigned hi = (unsigned) __double2hiint(x);
+	if (hi >= 0x40500000u) return exp_tab(-x, tab);
+	int m;
+	const unsigned long long e = pair_exp(pair_fix(hi, (unsigned) __double2loint(x)), m, ptab);
+	return pair_double(e, 63 + m);
+}
+
 // Kernel values of the gradient rows for centres multiplied by 1/w (c'), with the part of the derivative that varies
 // with the pair: dK/dc' = f cg (c_i' - c_j'), cg = K ('G'), K^2 ('C'), e^-r ('M'), f = -2, -2, -1
-template <typename T>
-__device__ __forceinline__ T cen_knl_grad(int type, T d2, T &cg, const double *tab)
+__device__ __forceinline__ double cen_knl_grad(int type, double d2, double &cg, const unsigned long long *ptab, const double *tab)
 {
-	if (type == 'G') return cg = exp_k(-d2, tab);
-	if (type == 'C') { const T k = rcp_nr((T) 1.0 + d2); cg = k * k; return k; }
-	T r = sqrt_k(d2), ex = exp_k(-r, tab);
-	cg = ex;
-	return fma(r, ex, ex);
+	if (type == 'G') return cg = exp_fix(d2, ptab, tab);
+	if (type == 'C') {
+		const double a = 1.0 + d2;
+		int m;
+		const unsigned long long v = pair_recip((unsigned) __double2hiint(a), (unsigned) __double2loint(a), m);
+		const double k = m < 62 ? pair_double(v, 63 + m) : 1.0 / a;
+		cg = k * k;
+		return k;
+	}
+	const unsigned long long r = pair_sqrt((unsigned) __double2hiint(d2), (unsigned) __double2loint(d2));
+	if (r == kPairFar) {
+		const double s = sqrt_nr(d2), ex = exp_tab(-s, tab);
+		cg = ex;
+		return fma(s, ex, ex);
+	}
+	int m;
+	const unsigned long long e = pair_exp(r, m, ptab);
+	cg = pair_double(e, 63 + m);
+	return pair_double(pair_mulh(r + (1ull << 57), e), 56 + m);
+}
+
+// the direction kernel and its derivative there; f = 2 / w^2
+__device__ __forceinline__ double dir_knl_grad(int type, double f, double ang, double &d1, const unsigned long long *ptab, const double *tab)
+{
+	if (type == 'B') { d1 = 2.0 * ang; return ang * ang; }
+	if (type == 'L') { d1 = 1.0; return ang; }
+	if (type == 'O') { const double k = exp_fix((1.0 - ang) * f, ptab, tab); d1 = k * f; return k; }
+	const double k = exp_fix(fma(-ang, ang, 1.0) * f, ptab, tab);     // 'U'
+	d1 = 2.0 * ang * (k * f);
+	return k;
 }
 
 // exp_tab and exp() (fn 0) or sqrt_nr and sqrt() (fn 1) side by side: accuracy check
@@ -286,6 +323,9 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 	__shared__ T sc[kVfdTile * D], su[kVfdTile * D], sv[kVfdTile], sl[kSplit ? kVfdTile * D : 1];
 	__shared__ double sc64[kN * kVfdTile * D + 1], su64[kN * kVfdTile * D + 1], sv64[kN * kVfdTile + 1];
 	__shared__ double sExp[(kSplit && !kNear) ? 1 : 256];
+	__shared__ unsigned long long sPair[kScaled && G ? 256 : 1];
+	if (kScaled && G)
+		for (int t = threadIdx.x; t < 256; t += blockDim.x) sPair[t] = c_pair_exp[t];
 	if (!kSplit || kNear)                                     // read after the tile barrier
 		for (int t = threadIdx.x; t < 256; t += blockDim.x) sExp[t] = c_exp2_256[t];
 	// work items (row block bx, column chunk cy), item = bx C + cy: with a queue, a persistent grid takes items
@@ -385,7 +425,7 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 					// per pair: t = K_c K_d v_j; centre part cg K_d v_j df; direction part b u_j with b = K_c K_d' v_j, and
 					// the row's own direction with weight t - b ang, i.e. tile - angSum at the end of the tile
 					T cg;
-					const T kc = cen_knl_grad<T>(ck, d2, cg, sExp), kd = dir_knl<T, true>(dk, diw2, ang, d1d, sExp);
+					const T kc = cen_knl_grad(ck, d2, cg, sPair, sExp), kd = dir_knl_grad(dk, (T) 2.0 * diw2, ang, d1d, sPair, sExp);
 					const T kv = kc * vj, cv = ck == 'G' ? kv * kd : (cg * vj) * kd, b = kv * d1d;
 					tile = fma(kv, kd, tile);
 					angSum = fma(b, ang, angSum);
@@ -452,35 +492,32 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 }
 
 // ---------------------------------------------------------------------------
-// The same row sums, without gradient, with the pair terms in fixed point (sa_pairfix.cuh): centre kernels 'M' and 'G',
-// direction kernels 'B' and 'L'.  A tile's directions and volumes are digits in the frame of its largest, its terms
-// are added in integers, and the sum is rounded to FP64 once per tile.
+// The same row sums, without gradient, with the pair terms in fixed point (sa_pairfix.cuh).  A tile's volumes, and its
+// directions for 'B' and 'L', are digits in the frame of its largest, its terms are added in integers, and the sum is
+// rounded to FP64 once per tile.  The arguments of 'O' and 'U' are formed in FP64.
 //
-// Two sets of 20 480 triangles, 'M' x 'B' (840 million pairs): 53.5 ms with the FP64 pair terms of k_vfd_rows (30 FP64 operations
-// a pair), 12.1 ms here; 580 clocks per pair and warp, of which the six FP64 operations of the squared distance take 384
-// and the rest is integer issue.  The other kernels ('C' needs a reciprocal, 'O' and 'U' a second exponential of either
-// sign) and gradient rows stay in FP64, as does the path without allocation.  Against 128-bit sums, 24 curves of 100 to
-// 1000 segments: root mean square error 2.1e-16 of the self term, FP64 pair terms 2.2e-16.
+// Two sets of 20 480 triangles, 'M' x 'B' (840 million pairs): 53.5 ms with the FP64 pair terms of k_vfd_rows (30 FP64
+// operations a pair), 12.1 ms here; 580 clocks per pair and warp, of which the six FP64 operations of the squared distance
+// take 384 and the rest is integer issue.  Against 128-bit sums, 24 curves of 100 to 1000 segments: root mean square
+// error 2.1e-16 of the self term, FP64 pair terms 2.2e-16.
 // ---------------------------------------------------------------------------
-__constant__ unsigned long long c_pair_exp[256] = {SA_PAIR_EXP_TABLE};
-
 struct __align__(16) PairColumn {
 	double2 c01;                              // centre in widths
 	double c2;
 	unsigned long long v;                     // volume at 63 bits, bit 63 its sign
-	int4 q0;                                  // direction digits: high 0, 1, 2, low 0
-	int2 q1;                                  // low 1, 2
-	int2 pad;
+	int4 q0;                                  // direction digits: high 0, 1, 2, low 0; 'O', 'U': components 0, 1
+	int4 q1;                                  // low 1, 2; component 2
 };
 
-template <int D, int CK>
-__global__ void __launch_bounds__(kVfdTile) k_vfd_rows_fix(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, double cw, int dk,
+// kProduct: 'B' and 'L'
+template <int D, int CK, bool kProduct>
+__global__ void __launch_bounds__(kVfdTile) k_vfd_rows_fix(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, double cw, int dk, double dw,
                                                            double *__restrict__ out, int symA, int C, int *__restrict__ queue)
 {
 	__shared__ PairColumn col[kVfdTile];
 	__shared__ unsigned long long tab[256];
 	__shared__ int sItem, sU[kVfdTile / 32], sV[kVfdTile / 32];
-	const double cs = 1.0 / cw;
+	const double cs = 1.0 / cw, f = 2.0 / (dw * dw);
 	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
 	for (int t = threadIdx.x; t < 256; t += kVfdTile) tab[t] = c_pair_exp[t];
 	const int rowBlocks = (R.n + kVfdTile - 1) / kVfdTile, nItems = rowBlocks * C;
@@ -539,8 +576,13 @@ __global__ void __launch_bounds__(kVfdTile) k_vfd_rows_fix(VfdSet R, VfdSet A, d
 					col[t].c2 = c[2];
 					col[t].v = (unsigned long long) __double2ll_rn(scalbn(fabs(v), 63 - eV)) |
 					           (__double2hiint(v) < 0 ? 1ull << 63 : 0ull);
-					col[t].q0 = make_int4(h[0], h[1], h[2], l[0]);
-					col[t].q1 = make_int2(l[1], l[2]);
+					if constexpr (kProduct) {
+						col[t].q0 = make_int4(h[0], h[1], h[2], l[0]);
+						col[t].q1 = make_int4(l[1], l[2], 0, 0);
+					} else {
+						*reinterpret_cast<double2 *>(&col[t].q0) = make_double2(u[0], u[1]);
+						*reinterpret_cast<double2 *>(&col[t].q1) = make_double2(u[2], 0.0);
+					}
 				}
 				__syncthreads();
 				if (act && (tileBad || bad)) acc = __longlong_as_double(0x7ff8000000000000ll);
@@ -548,28 +590,51 @@ __global__ void __launch_bounds__(kVfdTile) k_vfd_rows_fix(VfdSet R, VfdSet A, d
 					// sum of the terms as hi 2^32 + lo: 128 terms below 2^61
 					long long hi = 0, dg = 0;
 					unsigned long long lo32 = 0;
+					double large = 0.0, dgLarge = 0.0;       // terms with K_d > 1 (directions longer than 1)
 					for (int jj = sym ? max(0, i - j0) : 0; jj < nt; ++jj) {
 						const double2 c01 = col[jj].c01;
 						const double dx = ci[0] - c01.x, dy = ci[1] - c01.y;
 						double d2 = dx * dx + dy * dy;
 						if constexpr (D == 3) { const double dz = ci[2] - col[jj].c2; d2 = d2 + dz * dz; }
-						const int4 q0 = col[jj].q0;
-						const int2 q1 = col[jj].q1;
-						const int vh[3] = {q0.x, q0.y, q0.z}, vl[3] = {q0.w, q1.x, q1.y};
-						bool neg;
+						if constexpr (CK == 'C') d2 = 1.0 + d2;
 						int m;
-						const unsigned long long ang = pair_angle<D>(uh, ul, vh, vl, neg);
 						const unsigned long long kc = pair_centre(CK, (unsigned) __double2hiint(d2), (unsigned) __double2loint(d2), m, tab);
 						const unsigned long long w = col[jj].v;
-						long long s = (long long) pair_term(kc, m, dk, ang, w & ~(1ull << 63));
-						if ((neg && dk == 'L') != ((long long) w < 0)) s = -s;
+						const int4 q0 = col[jj].q0, q1 = col[jj].q1;
+						unsigned long long kd;
+						bool neg = false;
+						if constexpr (kProduct) {
+							const int vh[3] = {q0.x, q0.y, q0.z}, vl[3] = {q0.w, q1.x, q1.y};
+							kd = pair_angle<D>(uh, ul, vh, vl, neg);
+							if (dk == 'B') { kd = pair_mulh(kd, kd) << 1; neg = false; }
+						} else {
+							double ang = fma(ui[1], __hiloint2double(q0.w, q0.z), ui[0] * __hiloint2double(q0.y, q0.x));
+							if constexpr (D == 3) ang = fma(ui[2], __hiloint2double(q1.y, q1.x), ang);
+							const double x = (dk == 'O' ? 1.0 - ang : fma(-ang, ang, 1.0)) * f;   // K_d = e^-x
+							const unsigned xh = (unsigned) __double2hiint(x), xl = (unsigned) __double2loint(x);
+							if ((int) xh >= 0) {
+								int md;
+								kd = pair_exp(pair_fix(xh, xl), md, tab);
+								m += md;
+							} else if (xh < 0xbeb00000u) {   // x > -2^-20: unit vectors, rounding included
+								const unsigned long long y = pair_fix(xh & 0x7fffffffu, xl) << 6;
+								kd = (1ull << 63) + y + pair_mulh(y, y);
+							} else {
+								const double big = pair_double(kc, 63 + m) * exp(-x) * (pair_double(w & ~(1ull << 63), 2) * ((long long) w < 0 ? -1.0 : 1.0));
+								large += big;
+								if (sym && j0 + jj == i) dgLarge = big;
+								continue;
+							}
+						}
+						long long s = (long long) pair_term(kc, m, kd, w & ~(1ull << 63));
+						if (neg != ((long long) w < 0)) s = -s;
 						hi += s >> 32;
 						lo32 += (unsigned) s;
 						if (sym && j0 + jj == i) dg = s;
 					}
-					double ts = fma((double) hi, 0x1p32, (double) lo32);
-					if (sym) ts = 2.0 * ts - (double) dg;
-					acc += cv * scalbn(ts, (dk == 'B' ? 2 : 1) * (eRow + eU) + eV - 61);
+					double ts = fma((double) hi, 0x1p32, (double) lo32) + large;
+					if (sym) ts = 2.0 * ts - ((double) dg + dgLarge);
+					acc += cv * scalbn(ts, (kProduct ? (dk == 'B' ? 2 : 1) * (eRow + eU) : 0) + eV - 61);
 				}
 			}
 		}
@@ -853,14 +918,14 @@ static void launch_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet B, double cB, 
 	const int items = grid_for(R.n, kVfdBlock) * C;
 	SA_CHECK(cudaMemsetAsync(queue, 0, sizeof(int), s));
 	if constexpr (!G && sizeof(T) == sizeof(double)) {
-		if ((ck == 'M' || ck == 'G') && (dk == 'B' || dk == 'L')) {
-			auto kernel = ck == 'M' ? k_vfd_rows_fix<D, 'M'> : k_vfd_rows_fix<D, 'G'>;
-			kernel<<<vfd_grid((const void *) kernel, items), kVfdBlock, 0, s>>>(R, A, cA, B, cB, cw, dk, out, sym, C, queue);
-			return;
-		}
-	}
-	k_vfd_rows<D, T, G><<<vfd_grid((const void *) k_vfd_rows<D, T, G>, items), kVfdBlock, 0, s>>>(
-		R, A, cA, B, cB, ck, cw, dk, dw, out, dc, dt, sym, C, queue);
+		const bool product = dk == 'B' || dk == 'L';
+		auto kernel = ck == 'G' ? (product ? k_vfd_rows_fix<D, 'G', true> : k_vfd_rows_fix<D, 'G', false>)
+		            : ck == 'C' ? (product ? k_vfd_rows_fix<D, 'C', true> : k_vfd_rows_fix<D, 'C', false>)
+		                        : (product ? k_vfd_rows_fix<D, 'M', true> : k_vfd_rows_fix<D, 'M', false>);
+		kernel<<<vfd_grid((const void *) kernel, items), kVfdBlock, 0, s>>>(R, A, cA, B, cB, cw, dk, dw, out, sym, C, queue);
+	} else
+		k_vfd_rows<D, T, G><<<vfd_grid((const void *) k_vfd_rows<D, T, G>, items), kVfdBlock, 0, s>>>(
+			R, A, cA, B, cB, ck, cw, dk, dw, out, dc, dt, sym, C, queue);
 }
 
 // column chunks of the pair sums of a Vd x Vt objective: enough CTAs to fill the GPU (the pair sums are latency

@@ -24,15 +24,17 @@ def lib(tmp_path_factory):
     l = C.CDLL(out)
     l.pair_value.restype = C.c_double
     l.pair_value.argtypes = [C.c_int, C.c_int, C.c_double, C.c_void_p, C.c_void_p, C.c_double]
+    l.pair_exp.restype = C.c_double
+    l.pair_exp.argtypes = [C.c_double]
     l.pair_frame.argtypes = [C.c_double]
     return l
 
 
-@pytest.mark.parametrize("ck", "MG")
+@pytest.mark.parametrize("ck", "MGC")
 @pytest.mark.parametrize("dk", "BL")
 def test_error_bound(lib, ck, dk):
     rng = np.random.default_rng(ord(ck) + ord(dk))
-    lim = 4000.0 if ck == "M" else 63.0
+    lim = 63.0 if ck == "G" else 4000.0
     d2s = np.concatenate([[0.0, 5e-324, 1e-300, 1e-30, 0.25, np.nextafter(0.25, 0), 1.0, np.nextafter(1.0, 0), 4.0, lim,
                            np.nextafter(4096.0, 0), 4096.0, 1e5, 1e300], rng.uniform(0, 4, 300),
                           rng.uniform(0, lim, 300), 10.0 ** rng.uniform(-40, 3.5, 300)])
@@ -43,9 +45,9 @@ def test_error_bound(lib, ck, dk):
         if rng.uniform() < 0.2:
             w = u.copy()
         got = lib.pair_value(ord(ck), ord(dk), d2, u.ctypes.data, w.ctypes.data, v)
-        q = Decimal(float(d2))
+        q = Decimal(float(d2)) if ck != "C" else Decimal(1.0 + float(d2))
         r = q.sqrt()
-        k = (1 + r) * (-r).exp() if ck == "M" else (-q).exp()
+        k = (1 + r) * (-r).exp() if ck == "M" else (-q).exp() if ck == "G" else 1 / q
         a = sum(Decimal(float(x)) * Decimal(float(y)) for x, y in zip(u, w))
         t = k * (a * a if dk == "B" else a) * Decimal(float(v))
         bound = float(abs(t)) * (2.0 ** -54 + 2.0 ** -53) + float(k) * 2.0 ** -57 + 2.0 ** -61
@@ -58,3 +60,14 @@ def test_error_bound(lib, ck, dk):
 def test_frames(lib):
     for n2, e in ((1.0, 0), (1.0 + 1e-15, 0), (1.0 - 1e-15, 0), (1.01, 1), (0.26, 0), (0.25, -1), (4.0, 1), (4.1, 2)):
         assert lib.pair_frame(n2) == e and n2 <= 4.0 ** e * (1 + 2.0 ** -38)
+
+
+def test_exponential(lib):
+    """e^-x as a double for 0 <= x < 64: x itself is cut to 57 bits, the table and the polynomial lose 2^-58, the
+    conversion 2^-53: below 2^-52 together."""
+    rng = np.random.default_rng(2)
+    ln = np.log(2.0) / 256
+    x = np.concatenate([rng.uniform(0, 64, 2000), np.arange(0, 23000, 37) * ln, [0.0, 1e-300, 1e-17, 63.999999]])
+    for v in x:
+        t = (-Decimal(float(v))).exp()
+        assert abs(Decimal(lib.pair_exp(v)) / t - 1) < Decimal(2.0 ** -52), v

@@ -519,7 +519,8 @@ def main():
         pairs = float(Vd + Vt) ** 2
         t_obj = statistics.median(ts)
         evaluated = 0.5 * Vd * (Vd + 1) + float(Vd) * Vt      # symmetric DD half + DT; TT rows cached
-        objective = {"kernel": "k_vfd_rows (varifold pair sums, Matern-3/2 x Binet)", "deformed": Vd, "target": Vt,
+        objective = {"kernel": ("k_vfd_rows_fix" if args.precision == "fp64" else "k_vfd_rows") +
+                     " (varifold pair sums, Matern-3/2 x Binet)", "deformed": Vd, "target": Vt,
                      "pairs": pairs, "evaluated_pairs": evaluated, "ms": t_obj * 1e3, "pairs_per_s": pairs / t_obj,
                      "evaluated_pairs_per_s": evaluated / t_obj,
                      "what": "one sa_session_objective call (synchronous, host clock), median of 3 after one "
@@ -529,7 +530,8 @@ def main():
     value = ws * K / (ms_max / 1000.0)
     hbm, peak_kind = peaks()
     persistent = 0 < 4 * k_cnt < cg_iters              # one launch per solve, not one per iteration
-    kname = ("k_cg_persist (whole velocity CG solve: matvec, vector updates, dots)" if persistent
+    kname = (("k_cg_fix" if args.precision == "fp64" else "k_cg_persist") +
+             " (whole velocity CG solve: matvec, vector updates, dots)" if persistent
              else "k_cg_spmv (velocity block matvec + dot)")
     avg_launch_s = (k_ms / k_cnt) / 1000.0 if k_cnt else float("nan")
     N_, E_ = spec["lmkIniMat"].shape[1], spec["elmObj"]["elmVtxMat"].shape[1]
@@ -539,8 +541,8 @@ def main():
     bytes_per_launch = alg["iteration"] * iters_per_launch if persistent else alg["matvec"]
     achieved = bytes_per_launch / avg_launch_s / 1e9 if k_cnt else None
     traffic = None
-    tfile = os.path.join(ROOT, "profiles", ("k_cg_persist" if persistent else "k_cg_spmv") +
-                         f"_shell_l5_{args.precision}_traffic.txt")
+    tfile = os.path.join(ROOT, "profiles", (("k_cg_fix" if args.precision == "fp64" else "k_cg_persist") if persistent
+                                              else "k_cg_spmv") + f"_shell_l5_{args.precision}_traffic.txt")
     if os.path.exists(tfile) and args.workload == "shell":
         for line in open(tfile):
             if line.startswith("dram_bytes_per_iteration:") and cg_iters:
@@ -555,9 +557,9 @@ def main():
                                "(4 B x E) + 5 CG vectors (%d B x N x D) = %.2f MB" % (
                                    alg["elt"], alg["elt"], alg["iteration"] / 1e6),
                 "l2_operator_bytes_per_launch": k_bytes / k_cnt if k_cnt else None,
-                "l2_operator_note": "the kernel streams the assembled 3x3-block operator (values + column indices) "
-                                    "each iteration; it stays L2-resident (ncu: ~93% L2 hit), so these bytes are L2 "
-                                    "traffic, not HBM"}
+                "l2_operator_note": "the assembled 3x3-block operator (values, as digits on the FP64 path), read each "
+                                    "iteration: the part that stays in shared and tensor memory from there, the "
+                                    "rest from L2, so these bytes are on-chip traffic, not HBM"}
     # whole step, the same accounting (velocity CG + reaction-diffusion CG + per-step element passes)
     rd_iters = info["rdIterTotal"] - info0["rdIterTotal"]
     b_step = (cg_iters * alg["iteration"] + rd_iters * alg["rd_iteration"]) / K + alg["per_step"]
@@ -579,9 +581,12 @@ def main():
             "peak_source": "measured in this run: sa_selftest_fma_peak (independent FMA chains per thread, "
                            "256-thread CTAs, 2/4/8 CTAs per SM, best launch), its rate per SM clock x SMs x the "
                            "SM clock sampled during the timed steps",
-            "flops_model": "2 x (9 x operator slots + 10 x vector entries) per CG iteration (assembled 3x3 blocks; "
-                           "per entry the x, r, p, s updates, three dot terms and a row of the 3x3 block-Jacobi "
-                           "inverse)"}
+            "flops_model": ("2 x 10 x vector entries per CG iteration (per entry the x, r, p, s updates, three dot terms "
+                            "and a row of the 3x3 block-Jacobi inverse); the operator's products are summed on the "
+                            "integer pipes" if fp64 and persistent else
+                            "2 x (9 x operator slots + 10 x vector entries) per CG iteration (assembled 3x3 blocks; "
+                            "per entry the x, r, p, s updates, three dot terms and a row of the 3x3 block-Jacobi "
+                            "inverse)")}
 
     e2e = None
     if not args.no_e2e and rank == 0:

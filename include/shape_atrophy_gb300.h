@@ -49,11 +49,12 @@ extern "C" {
 #define SA_ELA_FRAME          0   /* reference frame elasticity, K-preconditioned CG */
 #define SA_ELA_ISOTROPIC      1   /* layered isotropic elasticity, block-Jacobi PCG */
 
-#define SA_PREC_FP64          0   /* all arithmetic in FP64 */
+#define SA_PREC_FP64          0   /* FP64, or fixed point of at least its precision (solver products, pair terms) */
 #define SA_PREC_MIXED         1   /* FP32 operators, FP64 dots/residuals + refinement */
 
-#define SA_CG_AUTO            0   /* persistent CG kernel (row state in registers when the grid fits one CTA
-                                     per SM, else vectors in global memory), two kernels when neither fits */
+#define SA_CG_AUTO            0   /* persistent CG kernel: FP64 block systems with fixed-point products when their plan
+                                     fits, else row state in registers when the grid fits one CTA per SM, else
+                                     vectors in global memory; two kernels when none fits */
 #define SA_CG_PERSISTENT      1   /* same as AUTO */
 #define SA_CG_TWO_KERNEL      2   /* matvec + vector kernel per iteration */
 #define SA_CG_PERSISTENT_GLOBAL 3 /* the persistent kernel with vectors in global memory at any size */

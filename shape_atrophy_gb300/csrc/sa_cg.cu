@@ -8,7 +8,11 @@
 // Chronopoulos-Gear form: per iteration one matvec w = A u with the dot
 // (w, u), and one update of p, s, x, r, u with the dots (r, u) and (r, r).
 // Stopping rule as the reference: |r|^2 < tol^2 |b|^2; b = 0 gives x = 0.
-// Four implementations of the same recurrences:
+// Five implementations of the same recurrences:
+//   k_cg_fix, k_cg_fix_many (sa_cgfix.cu)  the FP64 block systems' default:
+//                  as k_cg_persist, with the matrix products summed in
+//                  fixed point; a mesh its plan does not fit, and the
+//                  server, use the FP64 kernels below;
 //   k_cg_persist   one cooperative launch per solve, one CTA per SM, one
 //                  32-row slice per row warp with the row state in
 //                  registers, a reducer warp per CTA, the CTA's column
@@ -1378,7 +1382,8 @@ static CgScal run_cg(const Mesh &m, const TM *blk, const TV *dinv, const double 
 					// per iteration: operator digits once, u gathered once and written once; per launch: x, r, u in, x out
 					prof->profBytes += (double) h.iters * ((double) prof->plan.total * B * B * sizeof(TM) + 2.0 * sizeof(TV) * n) +
 					                   4.0 * sizeof(TV) * n;
-					prof->profFlops += (double) h.iters * 2.0 * ((double) B * B * m.slTotal + (7.0 + B) * n);
+					// FP64 only: the products run on the integer pipes
+					prof->profFlops += (double) h.iters * 2.0 * (7.0 + B) * n;
 				}
 				if (gaveUp || h.code == SA_ERR_TIMEOUT) throw DeviceWaitError{"persistent CG grid barrier"};
 				return h;

@@ -734,7 +734,7 @@ struct Stepper {
 		launch_assemble_elastic<D>(m, md, *gn, w.pd, w.blk, w.dinv, w.cw.binv64, w.cw.binv32, s);
 		launch_yank_rhs<D>(m, *gn, w.fy, w.b, s);
 		if (useK) {
-			if (!md.kernelFree) launch_kernel_matrix<D>(md, m.N, xn, w.K, s);
+			launch_kernel_matrix<D>(md, m.N, xn, w.K, w.kw, s);
 		} else if (md.precision == SA_PREC_MIXED)
 			k_to_f32<<<grid_for(m.slTotal * sell_vals<D>()), kBlock, 0, s>>>(m.slTotal * sell_vals<D>(), w.blk,
 			                                                                  w.cw.blk32);
@@ -1320,7 +1320,7 @@ static int adjoint_frame_impl(sa_context *ctx, Pool &P, Mesh &m, Model &md, cons
 			launch_adj_axpy(n, aXn, dt - 1.0, aXn, rhsV, s);
 			// velocity adjoint: (ldm K_t^{-1} + E_t) n = a_v, K-preconditioned CG started from K_t times the
 			// previous step's K^{-1} n
-			if (!md.kernelFree) launch_kernel_matrix<D>(md, m.N, xt, w.K, s);
+			launch_kernel_matrix<D>(md, m.N, xt, w.K, w.kw, s);
 			if (m.Bt > 0 && md.btmWgt != 0.0) launch_penalty_diag<D>(m, md, xt, w.pd, s);
 			launch_assemble_elastic<D>(m, md, w.g0, w.pd, w.blk, w.dinv, w.cw.binv64, nullptr, s);
 			code = kpcg<D>(m, md, w.blk, w.K, xt, rhsV, nu, w.kw, stt, &its, s);

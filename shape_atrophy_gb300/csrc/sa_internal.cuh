@@ -593,13 +593,16 @@ struct KpcgWork {
 	double *part, *scal;
 	int maxBlocks;
 	long partLen = 0;                     // doubles in part
+	int eA = 0;                           // frame of the RKHS matrix (launch_kernel_matrix)
+	int *over() const { return (int *) (scal + 24); }    // device: 2047 when an entry is not finite, else 0
 };
 // K: the stored kernel matrix, or null to evaluate it on the fly from the node positions q (interleaved)
 template <int D> int kpcg(const Mesh &m, const Model &md, const double *blk, const double *K, const double *q,
                           const double *b, double *x, KpcgWork &w, Status *st, int *itersOut, cudaStream_t s);
 // entries of the stored RKHS matrix (tiled, padded); two 28-bit digits each, the bytes of a double
 size_t kernel_matrix_entries(int N);
-template <int D> void launch_kernel_matrix(const Model &md, int N, const double *x, double *K, cudaStream_t s);
+// the RKHS matrix of a step: its frame, and its entries as digits unless K is null (evaluated in the products)
+template <int D> void launch_kernel_matrix(const Model &md, int N, const double *x, double *K, KpcgWork &w, cudaStream_t s);
 template <int D> void launch_adj_kernel_term(const Model &md, int N, const double *x, const double *alpha,
                                              const double *beta, double *ax, cudaStream_t s);
 

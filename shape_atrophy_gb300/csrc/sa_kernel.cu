@@ -438,13 +438,6 @@ constexpr int kKpLoad = 8;          // loads of a thread in flight (matrix entri
 constexpr int kKpFlush = 64;        // products per lane between flushes into 128 bits (kLimbMaxTerms at most)
 static_assert(kKpFlush <= kLimbMaxTerms, "digit sums would overflow");
 
-// the matrix's frame: exponent field of its largest entry
-static int kernel_frame(double eps)
-{
-	const double d = 1.0 + (eps > 0.0 ? eps : 0.0);
-	return fx_exp(d);
-}
-
 // The stored matrix is tiled: 8 rows x 4 columns per 256 bytes, the tiles of a row block one after the other, so that a
 // warp's load is two whole lines and the loads of a batch differ by constants.  Rows and columns past the end hold zero
 // entries.
@@ -459,11 +452,29 @@ size_t kernel_matrix_entries(int N)
 	return (size_t) ((N + kKpRows - 1) / kKpRows) * kernel_tiles(N) * 32;
 }
 
+// the largest exponent field of a matrix whose entries may exceed 1 (Matern kernels of a width that is not positive: k grows
+// with the distance there), into *e
+template <int D>
+__global__ void k_kernel_frame(int N, const double *__restrict__ x, int order, double w, double eps, int *e)
+{
+	int top = 1;
+	const long pairs = (long) N * N;
+	for (long k = blockIdx.x * (long) blockDim.x + threadIdx.x; k < pairs; k += (long) gridDim.x * blockDim.x) {
+		const int i = (int) (k / N), j = (int) (k - (long) i * N);
+		double v = kernel_entry<D>(order, w, load_node<D>(x, i), load_node<D>(x, j));
+		if (i == j) v += eps;
+		top = max(top, fx_exp(v));
+	}
+	top = fx_warp_max(top);
+	if ((threadIdx.x & 31) == 0) atomicMax(e, top);
+}
+
 // the matrix as digits: one thread per entry on or above the diagonal writes the mirrored entry too (the entries are
-// symmetric bit for bit)
+// symmetric bit for bit).  An entry above the frame is not finite (nodes that are not, widths that overflow): *over = 2047
+// then makes every product NaN.
 template <int D>
 __global__ void k_kernel_matrix_fix(int N, const double *__restrict__ x, int order, double w, double eps, int eA,
-                                    int2 *__restrict__ K)
+                                    int2 *__restrict__ K, int *over)
 {
 	const int lane = threadIdx.x & 31, ct = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 	if (ct >= kernel_tiles(N)) return;
@@ -480,6 +491,7 @@ __global__ void k_kernel_matrix_fix(int N, const double *__restrict__ x, int ord
 		if (i > j) continue;
 		double v = kernel_entry<D>(order, w, load_node<D>(x, i), qj);
 		if (i == j) v += eps;
+		if (fx_exp(v) > eA) atomicMax(over, 2047);
 		int2 t;
 		limb_matrix(v, eA, t.x, t.y);
 		K[kernel_place(N, i, j)] = t;
@@ -503,6 +515,7 @@ __device__ __forceinline__ Fx fx_xor_add(Fx f, int lanes)
 template <int D> struct KpSmem {
 	Fx seg[kKpPass][kKpWarps][D][kKpRows];
 	int e[kKpWarps];
+	int bad;                          // an entry evaluated in the product was above the frame
 };
 
 // first row block of CTA c: the blocks of kKpRows rows are dealt out evenly and contiguously
@@ -547,6 +560,7 @@ __device__ __forceinline__ void kernel_rows(int N, const int2 *__restrict__ K, c
 		for (int t = n + threadIdx.x; t < N * D; t += blockDim.x) e = max(e, fx_exp(__ldcg(r + t)));
 		e = fx_warp_max(e);
 		if (lane == 0) sm.e[wp] = e;
+		if (threadIdx.x == 0) sm.bad = 0;
 		__syncthreads();
 		eU = fx_warp_max(lane < W ? sm.e[lane] : 1);
 	}
@@ -581,6 +595,7 @@ __device__ __forceinline__ void kernel_rows(int N, const int2 *__restrict__ K, c
 						if (tile < t1 && i < N && j < N) {
 							double v = kernel_entry<D>(order, kw, qi, load_node<D>(q, j));
 							if (i == j) v += eps;
+							if (fx_exp(v) > eA) sm.bad = 1;
 							limb_matrix(v, eA, k[u].x, k[u].y);
 						}
 					}
@@ -647,7 +662,7 @@ __device__ __forceinline__ void kernel_rows(int N, const int2 *__restrict__ K, c
 			Fx s = fx_zero();
 #pragma unroll 4
 			for (int g = 0; g < kKpWarps; ++g) s = fx_add(s, sm.seg[b][g][d][a]);
-			const double v = eU >= 2047 || eA >= 2047 ? limb_bits(0x7FF8000000000000ull) : limb_round(s, eA + eU - 1020 + kKpRoom);
+			const double v = eU >= 2047 || eA >= 2047 || (kFree && sm.bad) ? limb_bits(0x7FF8000000000000ull) : limb_round(s, eA + eU - 1020 + kKpRoom);
 			if (i < N) out(i, d, v);
 		}
 		__syncthreads();
@@ -657,11 +672,12 @@ __device__ __forceinline__ void kernel_rows(int N, const int2 *__restrict__ K, c
 // y = K x, one launch (the products outside the persistent kernel)
 template <int D, bool kFree>
 __global__ void __launch_bounds__(32 * kKpWarps, 1)
-k_kernel_product(int N, const int2 *__restrict__ K, const double *__restrict__ q, int order, double kw, double eps, int eA,
-                 const double *x, double *y, int cap)
+k_kernel_product(int N, const int2 *__restrict__ K, const double *__restrict__ q, int order, double kw, double eps, int frame,
+                 const int *over, const double *x, double *y, int cap)
 {
 	extern __shared__ __align__(16) int2 kdig[];
 	__shared__ KpSmem<D> sm;
+	const int eA = max(frame, __ldg(over));
 	kernel_rows<D, kFree>(N, K, q, order, kw, eps, eA, x, kernel_block0(N, blockIdx.x, gridDim.x),
 	                      kernel_block0(N, blockIdx.x + 1, gridDim.x), kdig, cap, sm,
 	                      [&](int i, int d, double v) { y[(long) i * D + d] = v; });
@@ -742,7 +758,7 @@ constexpr int kKpColSlots = 4;      // slots of a warp whose columns are kept in
 template <int D, bool kFree>
 __global__ void __launch_bounds__(32 * kKpWarps, 1)
 k_kpcg_persist(SellOp A, const double *__restrict__ blk, const int2 *__restrict__ K, const double *__restrict__ q,
-               int order, double kw, double eps, int eA, KpVec v, double *part, KScal *sc, KpSums *ks, int cap)
+               int order, double kw, double eps, int frame, const int *over, KpVec v, double *part, KScal *sc, KpSums *ks, int cap)
 {
 	extern __shared__ __align__(16) int2 kdig[];
 	__shared__ FxScratch fs;
@@ -753,7 +769,7 @@ k_kpcg_persist(SellOp A, const double *__restrict__ blk, const int2 *__restrict_
 	__shared__ double rKr, rr, dAd, alpha, be;
 	__shared__ int sstate, code, it;
 	if (sc->done) return;                       // set before the launch: the same for every CTA
-	const int N = A.N, nctas = gridDim.x, lc = blockIdx.x;
+	const int N = A.N, nctas = gridDim.x, lc = blockIdx.x, eA = max(frame, __ldg(over));
 	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
 	// rows of phases A and B: 32-row slices dealt round-robin over the CTAs first, so that a small mesh
 	// spreads its row work (gathers) over all SMs instead of the first few CTAs
@@ -926,34 +942,40 @@ static void kpcg_persist_launch(const Mesh &m, const Model &md, const double *bl
 	SA_CHECK(cudaMemsetAsync(ks, 0, sizeof(KpSums), s));
 	SellOp A = sell_of(m);
 	KpVec v{x, wk.wK, wk.r, wk.Kr, wk.Kid, wk.dv, wk.dv2, wk.Ad};
-	int order = md.knlOrder, eA = kernel_frame(md.knlEps);
+	int order = md.knlOrder, eA = wk.eA;
+	const int *over = wk.over();
 	double kw = md.knlWidth, eps = md.knlEps;
 	double *part = wk.part;
-	void *args[] = {&A, (void *) &blk, (void *) &K, (void *) &q, &order, &kw, &eps, &eA, &v, &part, &sc, &ks, &cap};
+	void *args[] = {&A, (void *) &blk, (void *) &K, (void *) &q, &order, &kw, &eps, &eA, &over, &v, &part, &sc, &ks, &cap};
 	SA_CHECK(cudaLaunchCooperativeKernel((const void *) k_kpcg_persist<D, kFree>, dim3(nctas), dim3(32 * kKpWarps),
 	                                     args, bytes, s));
 }
 
 // y = K x with the digit matrix, or evaluated on the fly (K null)
 template <int D>
-static void kernel_product(const Model &md, int N, const int2 *K, const double *q, const double *x, double *y, cudaStream_t s)
+static void kernel_product(const Model &md, int N, const int2 *K, const double *q, const KpcgWork &wk, const double *x, double *y,
+                           cudaStream_t s)
 {
-	const int cap = kernel_dig_nodes<D>(N), eA = kernel_frame(md.knlEps);
+	const int cap = kernel_dig_nodes<D>(N);
 	const size_t bytes = sizeof(int2) * (size_t) D * cap;
 	const int nctas = std::min(device_sm_count(), (N + kKpRows - 1) / kKpRows);
-	if (K)
-		k_kernel_product<D, false><<<nctas, 32 * kKpWarps, bytes, s>>>(N, K, q, md.knlOrder, md.knlWidth, md.knlEps, eA, x, y, cap);
-	else
-		k_kernel_product<D, true><<<nctas, 32 * kKpWarps, bytes, s>>>(N, K, q, md.knlOrder, md.knlWidth, md.knlEps, eA, x, y, cap);
+	auto kernel = K ? k_kernel_product<D, false> : k_kernel_product<D, true>;
+	kernel<<<nctas, 32 * kKpWarps, bytes, s>>>(N, K, q, md.knlOrder, md.knlWidth, md.knlEps, wk.eA, wk.over(), x, y, cap);
 }
 
-// the RKHS matrix of a step, as digits
 template <int D>
-void launch_kernel_matrix(const Model &md, int N, const double *x, double *K, cudaStream_t s)
+void launch_kernel_matrix(const Model &md, int N, const double *x, double *K, KpcgWork &w, cudaStream_t s)
 {
+	SA_CHECK(cudaMemsetAsync(w.over(), 0, sizeof(int), s));
+	w.eA = limb_unit_frame(md.knlEps);
+	if (md.knlOrder >= 0 && !(md.knlWidth > 0.0)) {
+		k_kernel_frame<D><<<4 * device_sm_count(), 256, 0, s>>>(N, x, md.knlOrder, md.knlWidth, md.knlEps, w.over());
+		SA_CHECK(cudaMemcpyAsync(&w.eA, w.over(), sizeof(int), cudaMemcpyDeviceToHost, s));
+		SA_CHECK(cudaStreamSynchronize(s));
+	}
+	if (!K) return;
 	dim3 g(grid_for(kernel_tiles(N), 4), std::min((N + kKpRows - 1) / kKpRows, 65535));
-	k_kernel_matrix_fix<D><<<g, 128, 0, s>>>(N, x, md.knlOrder, md.knlWidth, md.knlEps, kernel_frame(md.knlEps),
-	                                         (int2 *) (void *) K);
+	k_kernel_matrix_fix<D><<<g, 128, 0, s>>>(N, x, md.knlOrder, md.knlWidth, md.knlEps, w.eA, (int2 *) (void *) K, w.over());
 }
 
 template <int D>
@@ -970,7 +992,7 @@ int kpcg(const Mesh &m, const Model &md, const double *blk, const double *K, con
 	SA_CHECK(cudaMemcpyAsync(sc, &h, sizeof(KScal), cudaMemcpyHostToDevice, s));
 	const int2 *Kfix = (const int2 *) (const void *) K;
 	const bool persist = kpcg_can_persist<D>(md, N);
-	auto product = [&](const double *in, double *out) { kernel_product<D>(md, N, Kfix, q, in, out, s); };
+	auto product = [&](const double *in, double *out) { kernel_product<D>(md, N, Kfix, q, wk, in, out, s); };
 	k_kp_bnorm<D><<<nb, kKBlock, 0, s>>>(N, b, wk.part, sc);
 	// warm start x0 = K w (w = K^{-1} v of the previous step)
 	product(wk.wK, x);
@@ -1008,8 +1030,8 @@ template void launch_adj_kernel_term<2>(const Model &, int, const double *, cons
                                         cudaStream_t);
 template void launch_adj_kernel_term<3>(const Model &, int, const double *, const double *, const double *, double *,
                                         cudaStream_t);
-template void launch_kernel_matrix<2>(const Model &, int, const double *, double *, cudaStream_t);
-template void launch_kernel_matrix<3>(const Model &, int, const double *, double *, cudaStream_t);
+template void launch_kernel_matrix<2>(const Model &, int, const double *, double *, KpcgWork &, cudaStream_t);
+template void launch_kernel_matrix<3>(const Model &, int, const double *, double *, KpcgWork &, cudaStream_t);
 template int kpcg<2>(const Mesh &, const Model &, const double *, const double *, const double *, const double *,
                      double *, KpcgWork &, Status *, int *, cudaStream_t);
 template int kpcg<3>(const Mesh &, const Model &, const double *, const double *, const double *, const double *,

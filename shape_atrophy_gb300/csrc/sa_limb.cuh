@@ -15,7 +15,9 @@
 //   sum va vu = 2^56 S2 + 2^28 S1 + S0, S2 = sum a1 u1, S1 = sum (a1 u0 + a0 u1), S0 = sum a0 u0, nothing dropped.  S1 is
 //     formed as M - S2 - S0 from M = sum (a1 + a0)(u1 + u0) (Karatsuba's product), so a product takes three integer
 //     multiply-adds, each about four clocks of a sub-partition, and two 32-bit additions.
-// Each sum stays below 2^63 for up to kLimbMaxTerms products.  An Inf or NaN in either factor gives NaN.
+// Each sum stays below 2^63 for up to kLimbMaxTerms products.  A frame of 2047 (an Inf or NaN in the row or the set) gives
+// NaN.  An entry above its frame has no digits (0 comes out): the caller's frame covers every entry, or the caller looks
+// for such entries and gives NaN.
 #pragma once
 #include "sa_fixsum.cuh"
 
@@ -28,8 +30,8 @@ SA_FX_HD void limb_matrix(double a, int eA, int &a1, int &a0)
 {
 	int e; unsigned long long m; bool neg;
 	fx_parts(a, e, m, neg);
-	const int d = eA - e;                                     // >= 0
-	const unsigned long long v = d < 64 ? (((m << 3) >> d) + 1ull) >> 1 : 0ull;
+	const int d = eA - e;                                     // >= 0 in the frame
+	const unsigned long long v = (unsigned) d < 64u ? (((m << 3) >> d) + 1ull) >> 1 : 0ull;
 	const long long s = neg ? -(long long) v : (long long) v;
 	const long long lo = ((s + (1ll << 27)) & ((1ll << 28) - 1)) - (1ll << 27);
 	a1 = (int) ((s - lo) >> 28);
@@ -41,12 +43,19 @@ SA_FX_HD void limb_vector(double u, int eU, int &u1, int &u0)
 {
 	int e; unsigned long long m; bool neg;
 	fx_parts(u, e, m, neg);
-	const int d = eU - e;                                     // >= 0
-	const unsigned long long v = d < 64 ? (((m << 4) >> d) + 1ull) >> 1 : 0ull;
+	const int d = eU - e;                                     // >= 0 in the frame
+	const unsigned long long v = (unsigned) d < 64u ? (((m << 4) >> d) + 1ull) >> 1 : 0ull;
 	const long long s = neg ? -(long long) v : (long long) v;
 	const int lo = (int) (((unsigned) s + (1u << 27)) & ((1u << 28) - 1u)) - (1 << 27);
 	u1 = (int) ((s - lo) >> 28);
 	u0 = lo;
+}
+
+// the frame of a matrix whose off-diagonal entries are 1 at most in size and whose diagonal entries are 1 + eps
+inline int limb_unit_frame(double eps)
+{
+	const int one = fx_exp(1.0), d = fx_exp(1.0 + eps);
+	return d > one ? d : one;
 }
 
 struct LimbSum { long long s2, sm, s0; };    // S2, M, S0

@@ -1209,35 +1209,11 @@ static void set_scal(CgScal *d, double tolSqu, int itrMax, double bb, cudaStream
 }
 
 // CTAs of k_cg_persist with `warps` warps each that can be resident at once (0: it cannot run)
-// largest dynamic shared memory of one k_cg_persist CTA (the device's opt-in limit less the kernel's static
-// shared memory), set as the kernel's limit on first use; 0 if that fails
-template <int B, typename TM, typename TV, typename TX>
-static size_t persist_smem_max()
-{
-	static std::mutex mu;                    // sessions and servers may size launches from several threads
-	static size_t lim = (size_t) -1;
-	std::lock_guard<std::mutex> lock(mu);
-	if (lim == (size_t) -1) {
-		lim = 0;
-		int dev = 0, optin = 0;
-		cudaFuncAttributes fa;
-		if (cudaGetDevice(&dev) == cudaSuccess &&
-		    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
-		    cudaFuncGetAttributes(&fa, k_cg_persist<B, TM, TV, TX>) == cudaSuccess && (size_t) optin > fa.sharedSizeBytes) {
-			const size_t want = (size_t) optin - fa.sharedSizeBytes;
-			if (cudaFuncSetAttribute(k_cg_persist<B, TM, TV, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			                         (int) want) == cudaSuccess)
-				lim = want;
-		}
-		cudaGetLastError();
-	}
-	return lim;
-}
-
 template <int B, typename TM, typename TV, typename TX>
 static int persist_capacity(int smCount, int warps, size_t smemBytes)
 {
-	if (warps < 1 || warps > kPersistMaxWarps || smemBytes > persist_smem_max<B, TM, TV, TX>()) return 0;
+	if (warps < 1 || warps > kPersistMaxWarps || smemBytes > smem_limit((const void *) k_cg_persist<B, TM, TV, TX>))
+		return 0;
 	int v = 0;
 	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_cg_persist<B, TM, TV, TX>, 32 * warps, smemBytes) !=
 	    cudaSuccess) {
@@ -1251,18 +1227,9 @@ static int persist_capacity(int smCount, int warps, size_t smemBytes)
 template <int B, typename TM, typename TV, typename TX>
 static int persist_g_capacity(int smCount, int warps, size_t smemBytes)
 {
-	static std::mutex mu;
-	static bool attr = false;
-	if (warps < 2 || warps > kPersistMaxWarps || smemBytes > (size_t) kColSmemMax) return 0;
-	std::lock_guard<std::mutex> lock(mu);
-	if (!attr) {
-		if (cudaFuncSetAttribute(k_cg_persist_g<B, TM, TV, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                         kColSmemMax) != cudaSuccess) {
-			cudaGetLastError();
-			return 0;
-		}
-		attr = true;
-	}
+	if (warps < 2 || warps > kPersistMaxWarps || smemBytes > (size_t) kColSmemMax ||
+	    smemBytes > smem_limit((const void *) k_cg_persist_g<B, TM, TV, TX>))
+		return 0;
 	int v = 0;
 	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_cg_persist_g<B, TM, TV, TX>, 32 * warps, smemBytes) !=
 	    cudaSuccess) {
@@ -1410,7 +1377,7 @@ static CgScal run_cg(const Mesh &m, const TM *blk, const TV *dinv, const double 
 	int kc = 0;
 	size_t dynSmem = colSmem;
 	if (sizeof(TM) == sizeof(float) && tabOk) {
-		const size_t lim = persist_smem_max<B, TM, TV, TX>(), perSlot = (size_t) pw * 32 * B * B * sizeof(TM);
+		const size_t lim = smem_limit((const void *) k_cg_persist<B, TM, TV, TX>), perSlot = (size_t) pw * 32 * B * B * sizeof(TM);
 		int widest = 0;
 		for (int sl = 0; sl < m.nslice; ++sl)
 			widest = std::max(widest, (m.slOffHost[sl + 1] - m.slOffHost[sl]) / 32);

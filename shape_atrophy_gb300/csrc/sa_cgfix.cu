@@ -22,7 +22,9 @@
 #include "sa_grid.cuh"
 #include "sa_limb.cuh"
 #include <algorithm>
+#include <map>
 #include <mutex>
+#include <utility>
 
 namespace sa {
 
@@ -142,22 +144,31 @@ __global__ void k_plan_columns(int P, int R, const int *__restrict__ rowPtr, con
 	}
 }
 
-static size_t fix_smem_limit(const void *kernel)
+size_t smem_limit(const void *kernel)
 {
-	int dev = 0, optin = 0;
+	static std::mutex mu;                    // sessions and servers may size launches from several threads
+	static std::map<std::pair<int, const void *>, size_t> known;     // the limit belongs to a device's copy of the kernel
+	int dev = 0;
+	if (cudaGetDevice(&dev) != cudaSuccess) {
+		cudaGetLastError();
+		return 0;
+	}
+	std::lock_guard<std::mutex> g(mu);
+	const auto at = known.find({dev, kernel});
+	if (at != known.end()) return at->second;
+	int optin = 0;
 	cudaFuncAttributes fa;
-	if (cudaGetDevice(&dev) != cudaSuccess ||
-	    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-	    cudaFuncGetAttributes(&fa, kernel) != cudaSuccess || (size_t) optin <= fa.sharedSizeBytes) {
-		cudaGetLastError();
-		return 0;
+	size_t want = 0;
+	if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+	    cudaFuncGetAttributes(&fa, kernel) == cudaSuccess && (size_t) optin > fa.sharedSizeBytes) {
+		want = (size_t) optin - fa.sharedSizeBytes;
+		if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) want) == cudaSuccess) {
+			known[{dev, kernel}] = want;
+			return want;
+		}
 	}
-	const size_t want = (size_t) optin - fa.sharedSizeBytes;
-	if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) want) != cudaSuccess) {
-		cudaGetLastError();
-		return 0;
-	}
-	return want;
+	cudaGetLastError();                      // not kept: the next call tries again
+	return 0;
 }
 
 bool cgfix_plan(const Mesh &m, const double *x0soa, int smCount, int maxWarps, CgPlan &p,
@@ -212,7 +223,7 @@ bool cgfix_plan(const Mesh &m, const double *x0soa, int smCount, int maxWarps, C
 	if (!p.lcol || !p.fix || !p.rowExp || !p.ug || !p.vec || (p.per > 1 && !p.pinv)) return false;
 	const int nw = (P + 31) / 32;
 	const size_t sm = sizeof(int) * (size_t) nw + sizeof(unsigned short) * (size_t) (nw + 1);
-	if (sm > 48 * 1024 && sm > fix_smem_limit((const void *) k_plan_columns)) return false;
+	if (sm > 48 * 1024 && sm > smem_limit((const void *) k_plan_columns)) return false;
 	k_plan_columns<<<p.nchunk, 512, sm, s>>>(P, R, m.rowPtr, m.femVtx + m.Z, p.perm, p.inv, p.width, p.off, p.haloCap,
 	                                         p.halo, p.haloNum, p.lcol);
 	SA_CHECK(cudaGetLastError());
@@ -1144,32 +1155,20 @@ bool cgfix_run(const Mesh &m, const double *blk, const double *binv, double *x, 
 {
 	const CgPlan &p = w.plan;
 	if (!p.ok || m.dim != B) return false;
-	static std::mutex mu;
-	static size_t limits[3];
-	static bool known = false;
-	{
-		std::lock_guard<std::mutex> g(mu);
-		if (!known) {
-			limits[0] = fix_smem_limit((const void *) k_cg_fix<B, false>);
-			limits[1] = fix_smem_limit((const void *) k_cg_fix<B, true>);
-			limits[2] = fix_smem_limit((const void *) k_cg_fix_many<B>);
-			known = true;
-		}
-	}
 	const int colMax = 32 * p.pw * p.widest;
 	const size_t perStage = (size_t) p.pw * (256 * B * B + 8);
 	int parts = 1, stages, per = p.per;
 	size_t smem;
 	const void *kernel;
 	if (per > 1) {
-		const size_t lim = limits[2], fixed = fix_many_smem<B>(p.pw, p.haloMax, 0);
+		const size_t lim = smem_limit((const void *) k_cg_fix_many<B>), fixed = fix_many_smem<B>(p.pw, p.haloMax, 0);
 		const size_t perStage = (size_t) p.pw * (many_slot<B>() + 8);
 		if (fixed + 2 * perStage > lim) return false;
 		stages = (int) ((lim - fixed) / perStage);
 		smem = fix_many_smem<B>(p.pw, p.haloMax, stages);
 		kernel = (const void *) k_cg_fix_many<B>;
 	} else {
-		const size_t lim = std::min(limits[0], limits[1]);
+		const size_t lim = std::min(smem_limit((const void *) k_cg_fix<B, false>), smem_limit((const void *) k_cg_fix<B, true>));
 		const bool resident = fix_smem<B>(p.pw, p.parts, p.haloMax, colMax, p.widest) <= lim;
 		parts = resident ? p.parts : 1;
 		const size_t fixed = fix_smem<B>(p.pw, parts, p.haloMax, colMax, 0);

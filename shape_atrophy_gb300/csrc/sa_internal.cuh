@@ -487,6 +487,10 @@ struct CgPlan {
 	double *pinv = nullptr;       // block inverses in that order (several chunks per CTA)
 };
 
+// largest dynamic shared memory of one CTA of a kernel on the current device (the opt-in limit less the kernel's static
+// shared memory), raised as the kernel's limit there on first use; 0 if that fails.  Any thread.
+size_t smem_limit(const void *kernel);
+
 struct CgWork {            // scratch of the Jacobi CG (Chronopoulos-Gear form)
 	double *r, *u, *w, *p, *sv;   // n each
 	double *part;                 // partial sums: 3 x maxBlocks

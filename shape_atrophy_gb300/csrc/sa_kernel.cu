@@ -19,7 +19,6 @@
 #include "sa_grid.cuh"
 #include "sa_limb.cuh"
 #include <algorithm>
-#include <mutex>
 #include <cmath>
 
 namespace sa {
@@ -901,31 +900,16 @@ static int device_sm_count()
 constexpr int kKpDigBytes = 160 * 1024;
 template <int D> static int kernel_dig_nodes(int N) { return std::min((N + 3) / 4 * 4, kKpDigBytes / (int) (4 * D * sizeof(int2)) * 4); }
 
-// digits of r in shared memory: the limit of both kernels, raised on first use
-template <int D, bool kFree>
-static void kp_smem()
-{
-	static std::mutex mu;
-	static bool done = false;
-	std::lock_guard<std::mutex> g(mu);
-	if (done) return;
-	SA_CHECK(cudaFuncSetAttribute(k_kpcg_persist<D, kFree>, cudaFuncAttributeMaxDynamicSharedMemorySize, kKpDigBytes));
-	SA_CHECK(cudaFuncSetAttribute(k_kernel_product<D, kFree>, cudaFuncAttributeMaxDynamicSharedMemorySize, kKpDigBytes));
-	done = true;
-}
-
 // whether the solves of this mesh can run as the persistent K-PCG
 template <int D>
 static bool kpcg_can_persist(const Model &md, int N)
 {
-	if (md.kernelFree) kp_smem<D, true>();
-	else kp_smem<D, false>();
 	if (md.cgKernel == SA_CG_TWO_KERNEL || device_sm_count() > kSumMaxCtas) return false;
 	const size_t bytes = sizeof(int2) * (size_t) D * kernel_dig_nodes<D>(N);
+	const void *kernel = md.kernelFree ? (const void *) k_kpcg_persist<D, true> : (const void *) k_kpcg_persist<D, false>;
+	if (bytes > smem_limit(kernel)) return false;
 	int occ = 0;
-	const cudaError_t e = md.kernelFree
-	    ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_kpcg_persist<D, true>, 32 * kKpWarps, bytes)
-	    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_kpcg_persist<D, false>, 32 * kKpWarps, bytes);
+	const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 32 * kKpWarps, bytes);
 	if (e != cudaSuccess) { cudaGetLastError(); return false; }
 	return occ >= 1;
 }
@@ -960,6 +944,7 @@ static void kernel_product(const Model &md, int N, const int2 *K, const double *
 	const size_t bytes = sizeof(int2) * (size_t) D * cap;
 	const int nctas = std::min(device_sm_count(), (N + kKpRows - 1) / kKpRows);
 	auto kernel = K ? k_kernel_product<D, false> : k_kernel_product<D, true>;
+	if (bytes > smem_limit((const void *) kernel)) throw CudaError{cudaErrorInvalidValue, "K product: shared memory"};
 	kernel<<<nctas, 32 * kKpWarps, bytes, s>>>(N, K, q, md.knlOrder, md.knlWidth, md.knlEps, wk.eA, wk.over(), x, y, cap);
 }
 

@@ -4,8 +4,10 @@
 // at 64 clocks per warp and SM sub-partition, 22 of the 35 us of an iteration on the 92 178-node shell, against
 // 6 us for reading the operator (94 MB) from the L2.  Here the products go through the integer pipes
 // (sa_limb.cuh), which takes them off the critical path and leaves the loads:
-//   * the operator is converted once per solve to two 28-bit digits per entry (k_cgfix_operator; the bytes of
-//     the FP64 entry).  A slice that fits its warp's ring of slots in shared memory stays there for the whole solve;
+//   * the solve runs on a scaled system (D^-1/2 A D^-1/2, powers of two; see the scales below), so that digits cut relative
+//     to a row's and a halo's largest entry lose nothing where soft and stiff materials meet;
+//   * the operator is converted once per solve to two digits per entry, of 28 and of up to 32 bits (k_cgfix_operator; the
+//     bytes of the FP64 entry).  A slice that fits its warp's ring of slots in shared memory stays there for the whole solve;
 //     of larger ones as many slots as fit stay in tensor memory (39 MB over the chip: with the operator, the vectors
 //     and u the working set of the shell is 107 MB, beyond what the L2 holds of a cyclic scan), and the rest is
 //     streamed by bulk copies into the ring, ahead of its use and across the grid barriers;
@@ -34,6 +36,11 @@ constexpr int kFixMaxParts = 8;            // warps per slice
 constexpr int kFixMaxHalo = 8192;          // halo nodes per chunk (shared memory takes about 6000 of them)
 constexpr int kFixStagers = 4;             // warps that stage at least, with several chunks per CTA
 constexpr int kFixMaxRows = 1 << 20;       // permuted rows whose bit map and prefix counts fit shared memory
+
+// the frame of a row of w 2^s and the exponent s of the row's scale in one word (both within 16 bits)
+__host__ __device__ __forceinline__ int row_pack(int e, int s) { return (int) ((unsigned) e << 16 | ((unsigned) s & 0xffffu)); }
+__host__ __device__ __forceinline__ int row_frame(int w) { return w >> 16; }
+__host__ __device__ __forceinline__ int row_scale(int w) { return (short) w; }
 
 template <int B> constexpr int limb_stride() { return 6; }    // words per halo node: three 8-byte bank pairs, odd, so consecutive nodes spread
 template <int B> constexpr int fix_u_stride() { return B == 3 ? 4 : 2; }   // doubles per node of the gather copy
@@ -217,10 +224,11 @@ bool cgfix_plan(const Mesh &m, const double *x0soa, int smCount, int maxWarps, C
 	p.lcol = (unsigned short *) get(sizeof(unsigned short) * (size_t) total);
 	p.fix = (int2 *) get(sizeof(int2) * (size_t) total * B * B);
 	p.rowExp = (int *) get(sizeof(int) * (size_t) P);
+	p.scale = (short *) get(sizeof(short) * (size_t) m.N);
 	p.ug = (double *) get(sizeof(double) * (size_t) P * (B == 3 ? fix_u_stride<3>() : fix_u_stride<2>()));
 	p.vec = (double *) get(sizeof(double) * (size_t) P * 4 * B);
 	if (p.per > 1) p.pinv = (double *) get(sizeof(double) * (size_t) P * B * B);
-	if (!p.lcol || !p.fix || !p.rowExp || !p.ug || !p.vec || (p.per > 1 && !p.pinv)) return false;
+	if (!p.lcol || !p.fix || !p.rowExp || !p.scale || !p.ug || !p.vec || (p.per > 1 && !p.pinv)) return false;
 	const int nw = (P + 31) / 32;
 	const size_t sm = sizeof(int) * (size_t) nw + sizeof(unsigned short) * (size_t) (nw + 1);
 	if (sm > 48 * 1024 && sm > smem_limit((const void *) k_plan_columns)) return false;
@@ -236,11 +244,46 @@ bool cgfix_plan(const Mesh &m, const double *x0soa, int smCount, int maxWarps, C
 }
 
 // ---------------------------------------------------------------------------
-// operator: the permuted rows' entries as digits, and the row frames.  One warp per slice.
+// Scales of a solve.  With D the block diagonal, the solve runs on D^-1/2 A D^-1/2, whose entries and whose u are alike in
+// soft and stiff materials: node i has the scale 2^s, the root of the largest entry of its block inverse to a power of two,
+// its u, p and x are over 2^s, its r, s and w times 2^s.  Powers of two, so the FP64 recurrences round as they would
+// without; (w, u) and (r, u) do not change, a row's share of (r, r) is taken back by 2^-2s.  With A and u as they are, and one
+// frame for a chunk's u, materials 1 : c : 1 on the icosphere-4 shell had errors of 5.1e-9 at c = 10^6 and 3.5e-6 at 10^8
+// (2,888 iterations); scaled, and with the operator's longer digits, 6.1e-11 and 6.0e-9 (2,323), as FP64 kernels among
+// themselves (9.6e-11, 6.1e-9, 2,345).
+// ---------------------------------------------------------------------------
+// v 2^s by the exponent field; zeros, subnormal numbers and results outside the normal range by scalbn
+__device__ __noinline__ double scale_edge(double v, int s) { return scalbn(v, s); }
+__device__ __forceinline__ double scale_pow2(double v, int s)
+{
+	const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff;
+	if (e != 0 && e != 2047 && e + s > 0 && e + s < 2047) return __hiloint2double(hi + s * (1 << 20), __double2loint(v));
+	return ((unsigned) hi << 1 | (unsigned) __double2loint(v)) == 0u ? v : scale_edge(v, s);
+}
+
+template <int B>
+__global__ void k_cgfix_gather_copy(int P, const int *__restrict__ perm, const double *__restrict__ u,
+                                    const double *__restrict__ binv, double *__restrict__ ug, short *__restrict__ scale)
+{
+	const int q = blockIdx.x * blockDim.x + threadIdx.x;
+	if (q >= P) return;
+	const int i = perm[q];
+	int e = 0;
+	if (i >= 0)
+		for (int t = 0; t < B * B; ++t) e = max(e, fx_exp(__ldg(binv + (long) i * (B * B) + t)));
+	const int s = i >= 0 && e < 2047 ? (e - 1023) >> 1 : 0;
+	if (i >= 0) scale[i] = (short) s;
+	for (int c = 0; c < fix_u_stride<B>(); ++c)
+		ug[(long) q * fix_u_stride<B>() + c] = i >= 0 && c < B ? scale_pow2(u[(long) i * B + c], -s) : 0.0;
+}
+
+// ---------------------------------------------------------------------------
+// operator: the permuted rows' scaled entries as digits, and the row frames.  One warp per slice.
 // ---------------------------------------------------------------------------
 template <int B>
 __global__ void __launch_bounds__(128) k_cgfix_operator(int nslice, SellOp A, const int *__restrict__ rowPtr,
                                                         const double *__restrict__ blk, const int *__restrict__ perm,
+                                                        const short *__restrict__ scale,
                                                         const int *__restrict__ width, const int *__restrict__ off,
                                                         int2 *__restrict__ fix, int *__restrict__ rowExp)
 {
@@ -248,30 +291,37 @@ __global__ void __launch_bounds__(128) k_cgfix_operator(int nslice, SellOp A, co
 	if (sl >= nslice) return;
 	const int i = perm[(long) sl * 32 + lane], w = width[sl];
 	const int len = i >= 0 ? rowPtr[i + 1] - rowPtr[i] : 0;
-	const double *row = blk + (i >= 0 ? ((long) __ldg(A.off + (i >> 5))) * (B * B) + (i & 31) : 0l);
-	int e = 1;
-	for (int k = 0; k < len; ++k)
-		for (int t = 0; t < B * B; ++t) e = max(e, fx_exp(__ldg(row + ((long) k * B * B + t) * 32)));
-	rowExp[(long) sl * 32 + lane] = e;
+	const long first = i >= 0 ? (long) __ldg(A.off + (i >> 5)) : 0l;
+	const double *row = blk + (i >= 0 ? first * (B * B) + (i & 31) : 0l);
+	const int *col = A.col + first + (i & 31);
+	const int own = i >= 0 ? __ldg(scale + i) : 0;
+	// the largest exponent, and the rows' sums of |a 2^s| 2^own (about 1 each) as FP32 numbers that are never too small
+	int e = kLimbNone;
+	float top = 0.0f, sum[B] = {};               // of the node's B rows, which share a frame
+#pragma unroll 2
+	for (int k = 0; k < len; ++k) {
+		const int s = __ldg(scale + __ldg(col + 32 * k));
+#pragma unroll
+		for (int t = 0; t < B * B; ++t) {
+			const double v = __ldg(row + ((long) k * B * B + t) * 32);
+			e = max(e, limb_scaled_exp(v, s));
+			const float f = limb_float_above(v, s + own);
+			top = fmaxf(top, f);
+			sum[t / B] += f;
+		}
+	}
+	for (int r = 1; r < B; ++r) sum[0] = fmaxf(sum[0], sum[r]);
+	if (e < kLimbBad) e -= limb_extra(top, sum[0], e + own);
+	rowExp[(long) sl * 32 + lane] = row_pack(e < kLimbBad ? e + own : kLimbBad, own);
 	int2 *o = fix + (long) off[sl] * (B * B) + lane;
-	for (int k = 0; k < w; ++k)
+	for (int k = 0; k < w; ++k) {
+		const int s = k < len ? __ldg(scale + __ldg(col + 32 * k)) : 0;
 		for (int t = 0; t < B * B; ++t) {
 			int2 d = make_int2(0, 0);
-			if (k < len && e < 2047) limb_matrix(__ldg(row + ((long) k * B * B + t) * 32), e, d.x, d.y);
+			if (k < len && e < kLimbBad) limb_matrix_wide(__ldg(row + ((long) k * B * B + t) * 32), e - s, d.x, d.y);
 			o[((long) k * B * B + t) * 32] = d;
 		}
-}
-
-// u (natural order, stride B) -> its gather copy in permuted order
-template <int B>
-__global__ void k_cgfix_gather_copy(int P, const int *__restrict__ perm, const double *__restrict__ u,
-                                    double *__restrict__ ug)
-{
-	const int q = blockIdx.x * blockDim.x + threadIdx.x;
-	if (q >= P) return;
-	const int i = perm[q];
-	for (int c = 0; c < fix_u_stride<B>(); ++c)
-		ug[(long) q * fix_u_stride<B>() + c] = i >= 0 && c < B ? u[(long) i * B + c] : 0.0;
+	}
 }
 
 // ---------------------------------------------------------------------------
@@ -463,7 +513,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 	const int o1 = worker ? __ldg(a.off + sl) : o0;
 	const char *src = (const char *) a.fix + (size_t) o1 * (8 * BB);
 	const unsigned short *mycol = scol + (o1 - o0) + lane;
-	const int eRow = rowWarp ? __ldg(a.rowExp + row) : 1;
+	const int rowWord = rowWarp ? __ldg(a.rowExp + row) : 0, scl = row_scale(rowWord);
 	const int nhalo = __ldg(a.haloNum + lc);
 	for (int t = threadIdx.x, n = __ldg(a.off + (lc + 1) * pw) - o0; t < n; t += blockDim.x) scol[t] = __ldg(a.lcol + o0 + t);
 	for (int t = threadIdx.x; t < nhalo; t += blockDim.x) shalo[t] = __ldg(a.halo + (long) lc * a.haloCap + t);
@@ -513,13 +563,13 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 #pragma unroll
 		for (int c = 0; c < B; ++c) {
 			const long k = (long) i * B + c;
-			g[32 * c] = own ? a.x[k] : 0.0;
+			g[32 * c] = own ? scale_pow2(a.x[k], -scl) : 0.0;
 			g[vs + 32 * c] = g[2 * vs + 32 * c] = 0.0;
-			g[3 * vs + 32 * c] = own ? a.r0[k] : 0.0;
-			su[32 * c] = own ? a.u0[k] : 0.0;
+			g[3 * vs + 32 * c] = own ? scale_pow2(a.r0[k], scl) : 0.0;
+			su[32 * c] = own ? scale_pow2(a.u0[k], -scl) : 0.0;
 		}
 		double *sbinv = (double *) (sdyn + oInv) + wp * BB * 32 + lane;
-		for (int t = 0; t < BB; ++t) sbinv[32 * t] = own ? __ldg(a.binv + (long) i * BB + t) : 0.0;
+		for (int t = 0; t < BB; ++t) sbinv[32 * t] = own ? scale_pow2(__ldg(a.binv + (long) i * BB + t), -2 * scl) : 0.0;
 	}
 	const int nst = 32 * (W - 1), nSt = reducer ? 0 : nhalo;    // the reducer warp stages nothing
 	unsigned target = 0;                         // arrivals of the partial-sum path
@@ -640,7 +690,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 			}
 			if (own) {
 #pragma unroll
-				for (int c = 0; c < B; ++c) wv[c] = limb_to_double(acc[c], eRow, eU);
+				for (int c = 0; c < B; ++c) wv[c] = limb_scaled_to_double(acc[c], row_frame(rowWord), eU);
 				d1 = wv[0] * su[0];
 				for (int c = 1; c < B; ++c) d1 += wv[c] * su[32 * c];
 			}
@@ -717,7 +767,8 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 			for (int c = 1; c < B; ++c) { d2[0] += rv[c] * uv[c]; d2[1] += rv[c] * rv[c]; }
 		}
 		const int fG[2] = {sum_frame(gam), sum_frame(rr)};
-		warp_digits<2>(d2, fG, dig[wp]);
+		const int fRow[2] = {fG[0], fG[1] + 2 * scl};    // r times 2^s
+		warp_digits<2>(d2, fRow, dig[wp]);
 		__syncthreads();
 		if (reducer) {
 			double t[2];
@@ -742,7 +793,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 		__syncthreads();
 		if (gaveUp) break;
 		if (slow) {
-			if (!slow_sum<2>(d2[0], d2[1], two, a.part + nctas, nctas, &a.gs->bar, target, fs)) {
+			if (!slow_sum<2>(d2[0], scalbn(d2[1], -2 * scl), two, a.part + nctas, nctas, &a.gs->bar, target, fs)) {
 				if (threadIdx.x == 0) gaveUp = 1;
 				__syncthreads();
 				break;
@@ -754,7 +805,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 	}
 	if (own)
 #pragma unroll
-		for (int c = 0; c < B; ++c) a.x[(long) i * B + c] = a.vec[vrow + 32 * c];
+		for (int c = 0; c < B; ++c) a.x[(long) i * B + c] = scale_pow2(a.vec[vrow + 32 * c], scl);
 	if (stream)                                  // the ring's copies in flight land before the CTA leaves
 		for (int k = 0; k < nstage; ++k) {
 			ring_wait(mb + 8 * stage, parity);
@@ -782,13 +833,14 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 // marked evict-first (a kept first chunk, or two, gave nothing more).
 // ---------------------------------------------------------------------------
 template <int B>
-__global__ void k_cgfix_inverses(int P, const int *__restrict__ perm, const double *__restrict__ binv, double *__restrict__ out)
+__global__ void k_cgfix_inverses(int P, const int *__restrict__ perm, const short *__restrict__ scale,
+                                 const double *__restrict__ binv, double *__restrict__ out)
 {
 	const int q = blockIdx.x * blockDim.x + threadIdx.x;
 	if (q >= P) return;
 	const int i = perm[q];
 	for (int t = 0; t < B * B; ++t)
-		out[(long) (q >> 5) * (32 * B * B) + 32 * t + (q & 31)] = i >= 0 ? binv[(long) i * (B * B) + t] : 0.0;
+		out[(long) (q >> 5) * (32 * B * B) + 32 * t + (q & 31)] = i >= 0 ? scale_pow2(binv[(long) i * (B * B) + t], -2 * scale[i]) : 0.0;
 }
 
 // bytes of a ring slot: entries and columns
@@ -893,14 +945,14 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix_many(const FixA
 		open_chunk();
 		for (int k = 0; k < nstage; ++k) load_next(k);
 		for (int j = 0; j < per; ++j) {
-			const int row = (sl0 + j * pw) * 32 + lane, i = __ldg(a.perm + row);
+			const int row = (sl0 + j * pw) * 32 + lane, i = __ldg(a.perm + row), scl = row_scale(__ldg(a.rowExp + row));
 			double *g = a.vec + (long) (sl0 + j * pw) * 32 * B + lane;
 #pragma unroll
 			for (int c = 0; c < B; ++c) {
 				const long k = (long) i * B + c;
-				g[32 * c] = i >= 0 ? a.x[k] : 0.0;
+				g[32 * c] = i >= 0 ? scale_pow2(a.x[k], -scl) : 0.0;
 				g[vs + 32 * c] = g[2 * vs + 32 * c] = 0.0;
-				g[3 * vs + 32 * c] = i >= 0 ? a.r0[k] : 0.0;
+				g[3 * vs + 32 * c] = i >= 0 ? scale_pow2(a.r0[k], scl) : 0.0;
 			}
 		}
 	}
@@ -972,7 +1024,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix_many(const FixA
 				const int sl = sl0 + j * pw, row = sl * 32 + lane, nr = ring_slots(j), nt = j == 0 ? ntm : 0;
 				const int *uh = slimb + (j & 1) * a.haloMax * S;
 				const bool own = __ldg(a.perm + row) >= 0;
-				const int eRow = __ldg(a.rowExp + row);
+				const int rowWord = __ldg(a.rowExp + row);
 				double *g = a.vec + vs + (long) sl * 32 * B + lane;
 				double uv[B], pv[B], sv[B];
 				load_halo<B>(a.ug + (long) row * U, uv);
@@ -1007,7 +1059,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix_many(const FixA
 					const double be = beta;
 #pragma unroll
 					for (int c = 0; c < B; ++c) {
-						const double w = limb_to_double(acc[c], eRow, eU);
+						const double w = limb_scaled_to_double(acc[c], row_frame(rowWord), eU);
 						d1 += w * uv[c];
 						g[32 * c] = uv[c] + be * pv[c];
 						g[vs + 32 * c] = w + be * sv[c];
@@ -1071,6 +1123,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix_many(const FixA
 				double *g = a.vec + 2 * vs + (long) sl * 32 * B + lane;
 				const double *mi = a.pinv + (long) sl * 32 * BB + lane;
 				double rv[B], sv[B], uv[B], m[BB];
+				const double back = __hiloint2double((1023 - 2 * row_scale(__ldg(a.rowExp + sl * 32 + lane))) << 20, 0);   // 2^-2s
 #pragma unroll
 				for (int c = 0; c < B; ++c) { rv[c] = g[vs + 32 * c]; sv[c] = g[32 * c]; }
 #pragma unroll
@@ -1087,8 +1140,11 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix_many(const FixA
 				double2 *o = reinterpret_cast<double2 *>(a.ug + (long) (sl * 32 + lane) * U);
 				o[0] = make_double2(uv[0], uv[1]);
 				if constexpr (B == 3) o[1] = make_double2(uv[2], 0.0);
+				double q = rv[0] * rv[0];
+				d2[0] += rv[0] * uv[0];
 #pragma unroll
-				for (int c = 0; c < B; ++c) { d2[0] += rv[c] * uv[c]; d2[1] += rv[c] * rv[c]; }
+				for (int c = 1; c < B; ++c) { d2[0] += rv[c] * uv[c]; q += rv[c] * rv[c]; }
+				d2[1] = fma(q, back, d2[1]);
 			}
 		const int fG[2] = {sum_frame(gam), sum_frame(rr)};
 		warp_digits<2>(d2, fG, dig[wp]);
@@ -1131,11 +1187,11 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix_many(const FixA
 	}
 	if (rowWarp) {
 		for (int j = 0; j < per; ++j) {
-			const int i = __ldg(a.perm + (sl0 + j * pw) * 32 + lane);
+			const int row = (sl0 + j * pw) * 32 + lane, i = __ldg(a.perm + row), scl = row_scale(__ldg(a.rowExp + row));
 			const double *g = a.vec + (long) (sl0 + j * pw) * 32 * B + lane;
 			if (i >= 0)
 #pragma unroll
-				for (int c = 0; c < B; ++c) a.x[(long) i * B + c] = g[32 * c];
+				for (int c = 0; c < B; ++c) a.x[(long) i * B + c] = scale_pow2(g[32 * c], scl);
 		}
 		for (int k = 0; k < nstage; ++k) {       // the ring's copies in flight land before the CTA leaves
 			ring_wait(mb + 8 * stage, parity);
@@ -1185,10 +1241,10 @@ bool cgfix_run(const Mesh &m, const double *blk, const double *binv, double *x, 
 	}
 	if (nctas > occ * w.smCount || nctas > kSumMaxCtas) return false;
 	const int P = p.nchunk * 32 * p.pw;
-	k_cgfix_operator<B><<<(p.nslice + 3) / 4, 128, 0, s>>>(p.nslice, sell_of(m), m.rowPtr, blk, p.perm, p.width, p.off,
-	                                                       p.fix, p.rowExp);
-	k_cgfix_gather_copy<B><<<grid_for(P), kBlock, 0, s>>>(P, p.perm, u, p.ug);
-	if (per > 1) k_cgfix_inverses<B><<<grid_for(P), kBlock, 0, s>>>(P, p.perm, binv, p.pinv);
+	k_cgfix_gather_copy<B><<<grid_for(P), kBlock, 0, s>>>(P, p.perm, u, binv, p.ug, p.scale);
+	k_cgfix_operator<B><<<(p.nslice + 3) / 4, 128, 0, s>>>(p.nslice, sell_of(m), m.rowPtr, blk, p.perm, p.scale,
+	                                                       p.width, p.off, p.fix, p.rowExp);
+	if (per > 1) k_cgfix_inverses<B><<<grid_for(P), kBlock, 0, s>>>(P, p.perm, p.scale, binv, p.pinv);
 	SA_CHECK(cudaMemsetAsync(w.bar, 0, sizeof(GridSums), s));
 	FixArgs a{p.pw, parts, p.haloCap, p.haloMax, colMax, stages, p.perm, p.width, p.off, p.halo, p.haloNum, p.rowExp, p.lcol, p.fix,
 	          binv, r, u, x, p.ug, p.vec, w.part, p.pinv, (CgScal *) w.scal, (GridSums *) w.bar};

@@ -480,11 +480,12 @@ struct CgPlan {
 	int *width = nullptr, *off = nullptr;   // nslice (+ 1): longest row and first slot of each 32-row slice
 	unsigned short *lcol = nullptr;         // total: place of each slot's column in its chunk's halo list
 	int *halo = nullptr, *haloNum = nullptr;   // nchunk x haloCap permuted rows, and their count per chunk
+	short *scale = nullptr;       // N: exponent of each node's scale, per solve
 	int2 *fix = nullptr;          // total x B x B: the operator's entries as two digits
-	int *rowExp = nullptr;        // nchunk 32 pw: largest exponent field of each permuted row
-	double *ug = nullptr;         // the gather copy of u in permuted order (3-component nodes padded to 4)
-	double *vec = nullptr;        // x, p, s and r of the permuted rows, [vector][slice][component][lane]
-	double *pinv = nullptr;       // block inverses in that order (several chunks per CTA)
+	int *rowExp = nullptr;        // nchunk 32 pw: frame of each permuted row's scaled entries, and the row's scale again
+	double *ug = nullptr;         // the gather copy of u over its scales in permuted order (3-component nodes padded to 4)
+	double *vec = nullptr;        // scaled x, p, s and r of the permuted rows, [vector][slice][component][lane]
+	double *pinv = nullptr;       // scaled block inverses in that order (several chunks per CTA)
 };
 
 // largest dynamic shared memory of one CTA of a kernel on the current device (the opt-in limit less the kernel's static

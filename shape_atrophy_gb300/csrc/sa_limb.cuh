@@ -136,6 +136,87 @@ double limb_round(Fx f, int em)
 	return limb_bits(bits | (neg ? 1ull << 63 : 0ull));
 }
 
+// Column scales.  Where columns differ much in size (a stiff layer beside a soft one: rows of A of 10^6 beside 1, u = A^-1 r
+// the other way round), one frame for all of u would round the small entries that the large rows multiply.  So each
+// column has a power of two, 2^s: the sum is that of (a 2^s)(u 2^-s) and the frames are those of the scaled entries.  The
+// matrix's digits are cut from the entries as they are, in the frame eA - s; u comes scaled.
+constexpr int kLimbBad = 1 << 14, kLimbNone = -(1 << 14);     // frames of a set with an Inf or NaN, of zeros only
+
+// exponent field of v 2^s
+SA_FX_HD int limb_scaled_exp(double v, int s)
+{
+	unsigned long long b;
+#if defined(__CUDA_ARCH__)
+	b = (unsigned long long) __double_as_longlong(v);
+#else
+	__builtin_memcpy(&b, &v, 8);
+#endif
+	const int e = (int) (b >> 52 & 0x7FFull);
+	return e >= 2047 ? kLimbBad : b << 1 ? (e > 1 ? e : 1) + s : kLimbNone;
+}
+
+// an FP32 number of at least |v 2^s|, from 2^-126 on: a normal v rounded up (infinite beyond the range)
+SA_FX_HD float limb_float_above(double v, int s)
+{
+	unsigned long long b;
+#if defined(__CUDA_ARCH__)
+	b = (unsigned long long) __double_as_longlong(v);
+#else
+	__builtin_memcpy(&b, &v, 8);
+#endif
+	const int e = (int) (b >> 52 & 0x7FFull) + s - 896;       // FP32 field
+	const unsigned m = ((unsigned) (b >> 29) & 0x7FFFFFu) + 1u;
+	const unsigned f = e > 253 ? 0x7F800000u : e < 1 ? 0x00800000u : ((unsigned) e << 23) + m;
+#if defined(__CUDA_ARCH__)
+	return __uint_as_float(f);
+#else
+	float r;
+	__builtin_memcpy(&r, &f, 4);
+	return r;
+#endif
+}
+
+// More bits for a whole row at once: rows of an operator have few large entries, so their digits may be up to 2^4 longer
+// than limb_matrix's before a digit sum leaves 63 bits.  The bits that a row can take, from its largest |a 2^s| (top) and the
+// sum of them, both 2^x of what they are, and its frame e, x included.  With 80 products of |u1 + u0| <= 1.5 2^28 and
+// |a0| <= 2^27, |a1| may sum to 2^33.4 (a1 = a 2^(1049 - e)); a1 + a0 stays a 32-bit number.
+constexpr int kLimbExtra = 4;
+SA_FX_HD int limb_extra(float top, float sum, int e)
+{
+	if (e < 1023 - 100 || e > 1023 + 100) return 0;
+	const unsigned bits = (unsigned) (127 + 1023 - e) << 23; // 2^(1023 - e)
+	float unit;
+#if defined(__CUDA_ARCH__)
+	unit = __uint_as_float(bits);
+#else
+	__builtin_memcpy(&unit, &bits, 4);
+#endif
+	const float t = top * unit, m = sum * unit;              // of |a1|, in units of 2^26
+	int g = 0;
+	while (g < kLimbExtra && t * (float) (2 << g) <= 29.9f && m * (float) (2 << g) <= 163.0f) ++g;
+	return g;
+}
+
+// limb_matrix in a frame up to kLimbExtra below the entry's exponent
+SA_FX_HD void limb_matrix_wide(double a, int eA, int &a1, int &a0)
+{
+	int e; unsigned long long m; bool neg;
+	fx_parts(a, e, m, neg);
+	const int d = eA - e;                                     // >= -kLimbExtra
+	const unsigned long long v = d < 0 ? (d >= -kLimbExtra ? m << (2 - d) : 0ull) : d < 64 ? (((m << 3) >> d) + 1ull) >> 1 : 0ull;
+	const long long s = neg ? -(long long) v : (long long) v;
+	const long long lo = ((s + (1ll << 27)) & ((1ll << 28) - 1)) - (1ll << 27);
+	a1 = (int) ((s - lo) >> 28);
+	a0 = (int) lo;
+}
+
+// the sum as a double, for the frames of the scaled entries
+SA_FX_HD double limb_scaled_to_double(const LimbSum &t, int eA, int eU)
+{
+	if (eA >= kLimbBad || eU >= 2047) return limb_bits(0x7FF8000000000000ull);
+	return limb_round(limb_fixed(t), eA + eU - 1020);
+}
+
 // the sum as a double, for the matrix frame eA and the vector frame eU
 SA_FX_HD double limb_to_double(const LimbSum &t, int eA, int eU)
 {

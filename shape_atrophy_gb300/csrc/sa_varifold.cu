@@ -201,7 +201,10 @@ __device__ __forceinline__ T dir_knl(int type, T iw2, T ang, T &d1, const double
 
 // The gradient rows' FP64 work per pair is what bounds them (5120 x 5120 triangles, 'C' x 'O': 12.1 -> 7.2 ms a call when
 // the divisions, the width scalings and the row factors left the pair loop, 4.3 ms when the kernel values were
-// formed in fixed point, sa_pairfix.cuh, and converted).
+// formed in fixed point, sa_pairfix.cuh, and converted).  Two sums stay pair by pair although they cost more there: centre
+// differences of centres as they are, which are exact between near elements (centres over w first: 1.3 to 1.7 times the
+// gradient's error ten and more shape sizes from the origin), and the part of u_j across u_i, b (u_j - ang u_i), which is small
+// where sum(b u_j) and u_i sum(b ang) are not (up to 2.8 times the error, 'O' and 'U' kernels).  Both together: 4.25 -> 4.44 ms.
 // e^-x; outside [0, 64) by exp_tab
 __device__ __forceinline__ double exp_fix(double x, const unsigned long long *ptab, const double *tab)
 {
@@ -212,22 +215,25 @@ __device__ __forceinline__ double exp_fix(double x, const unsigned long long *pt
 	return pair_double(e, 63 + m);
 }
 
-// Kernel values of the gradient rows for centres multiplied by 1/w (c'), with the part of the derivative that varies
-// with the pair: dK/dc' = f cg (c_i' - c_j'), cg = K ('G'), K^2 ('C'), e^-r ('M'), f = -2, -2, -1
-__device__ __forceinline__ double cen_knl_grad(int type, double d2, double &cg, const unsigned long long *ptab, const double *tab)
+// Kernel values of the gradient rows, q = d2 / w^2 the squared distance in widths (d2 unscaled, iw2 = 1 / w^2), with the part
+// of the derivative that varies with the pair: dK/dc_i = f cg (c_i - c_j) / w^2, cg = K ('G'), K^2 ('C'), e^-r ('M'),
+// f = -2, -2, -1
+__device__ __forceinline__ double cen_knl_grad(int type, double d2, double iw2, double &cg, const unsigned long long *ptab,
+                                               const double *tab)
 {
-	if (type == 'G') return cg = exp_fix(d2, ptab, tab);
+	if (type == 'G') return cg = exp_fix(d2 * iw2, ptab, tab);
 	if (type == 'C') {
-		const double a = 1.0 + d2;
+		const double a = fma(d2, iw2, 1.0);
 		int m;
 		const unsigned long long v = pair_recip((unsigned) __double2hiint(a), (unsigned) __double2loint(a), m);
 		const double k = m < 62 ? pair_double(v, 63 + m) : 1.0 / a;
 		cg = k * k;
 		return k;
 	}
-	const unsigned long long r = pair_sqrt((unsigned) __double2hiint(d2), (unsigned) __double2loint(d2));
+	const double q = d2 * iw2;
+	const unsigned long long r = pair_sqrt((unsigned) __double2hiint(q), (unsigned) __double2loint(q));
 	if (r == kPairFar) {
-		const double s = sqrt_nr(d2), ex = exp_tab(-s, tab);
+		const double s = sqrt_nr(q), ex = exp_tab(-s, tab);
 		cg = ex;
 		return fma(s, ex, ex);
 	}
@@ -316,15 +322,15 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 	// cancellation DD - 2 DT + TT).
 	constexpr bool kNear = kSplit && !G;
 	constexpr int kN = kNear ? 1 : 0;
-	// FP64: centres (rows and tiles) multiplied by 1/w as they are loaded, so the pair term does not scale the squared
-	// distance (the gradient's centre derivatives are multiplied by 1/w once per row)
-	constexpr bool kScaled = !kSplit;
+	// FP64 objective: centres (rows and tiles) multiplied by 1/w as they are loaded, so the pair term does not
+	// scale the squared distance (the gradient keeps unscaled centres, see cen_knl_grad)
+	constexpr bool kScaled = !kSplit && !G, kFixG = !kSplit && G;
 	const double cs = kScaled ? 1.0 / cw : 1.0;
 	__shared__ T sc[kVfdTile * D], su[kVfdTile * D], sv[kVfdTile], sl[kSplit ? kVfdTile * D : 1];
 	__shared__ double sc64[kN * kVfdTile * D + 1], su64[kN * kVfdTile * D + 1], sv64[kN * kVfdTile + 1];
 	__shared__ double sExp[(kSplit && !kNear) ? 1 : 256];
-	__shared__ unsigned long long sPair[kScaled && G ? 256 : 1];
-	if (kScaled && G)
+	__shared__ unsigned long long sPair[kFixG ? 256 : 1];
+	if (kFixG)
 		for (int t = threadIdx.x; t < 256; t += blockDim.x) sPair[t] = c_pair_exp[t];
 	if (!kSplit || kNear)                                     // read after the tile barrier
 		for (int t = threadIdx.x; t < 256; t += blockDim.x) sExp[t] = c_exp2_256[t];
@@ -400,7 +406,7 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 			// tile = sum of K_c K_d vol_j over the tile's columns; the row factor coef * vol_i and, for the
 			// symmetric half, the weights (2 off the diagonal, 1 on it: 2 tile - diagonal term) are applied
 			// once per tile
-			T tile = 0, comp = 0, diag = 0, angSum = 0, tgc[D], tgt[D];
+			T tile = 0, comp = 0, diag = 0, tgc[D], tgt[D];
 			double nearSum = 0.0, diag64 = 0.0;                       // FP64 near-field terms (kNear)
 			for (int d = 0; d < D; ++d) { tgc[d] = 0; tgt[d] = 0; }
 			for (int jj = 0; jj < nt; ++jj) {
@@ -421,17 +427,16 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 				for (int d = 1; d < D; ++d) ang = ang + ui[d] * su[jj * D + d];
 				T d1c = 0, d1d = 0;
 				T vj = sv[jj];
-				if constexpr (kScaled && G) {
-					// per pair: t = K_c K_d v_j; centre part cg K_d v_j df; direction part b u_j with b = K_c K_d' v_j, and
-					// the row's own direction with weight t - b ang, i.e. tile - angSum at the end of the tile
+				if constexpr (kFixG) {
+					// per pair: t = K_c K_d v_j; centre part cg K_d v_j df; direction part b (u_j - ang u_i) with b = K_c K_d' v_j,
+					// and the row's own direction with weight t, i.e. tile at the end of the tile
 					T cg;
-					const T kc = cen_knl_grad(ck, d2, cg, sPair, sExp), kd = dir_knl_grad(dk, (T) 2.0 * diw2, ang, d1d, sPair, sExp);
+					const T kc = cen_knl_grad(ck, d2, ciw2, cg, sPair, sExp), kd = dir_knl_grad(dk, (T) 2.0 * diw2, ang, d1d, sPair, sExp);
 					const T kv = kc * vj, cv = ck == 'G' ? kv * kd : (cg * vj) * kd, b = kv * d1d;
 					tile = fma(kv, kd, tile);
-					angSum = fma(b, ang, angSum);
 					for (int d = 0; d < D; ++d) {
 						tgc[d] = fma(cv, df[d], tgc[d]);
-						tgt[d] = fma(b, su[jj * D + d], tgt[d]);
+						tgt[d] = fma(b, fma(-ang, ui[d], su[jj * D + d]), tgt[d]);
 					}
 					continue;
 				}
@@ -471,12 +476,12 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 			// Kahan: the FP32 sum with its lost low part, plus the FP64 near-field terms
 			const double tsum = ((double) tile - (double) comp) + nearSum;
 			acc += cv * (sym ? 2.0 * tsum - ((double) diag + diag64) : tsum);
-			if (kScaled && G) {
-				// centre part times f / w and the row's weights (cen_knl_grad); directions: D = 2: v = |e|, D = 3: v = |n| / 2
-				const double fc = (double) gco * (double) vi * cs * (ck == 'M' ? -1.0 : -2.0), ft = (double) gco * (double) half;
+			if (kFixG) {
+				// centre part times f / w^2 and the row's weights (cen_knl_grad); directions: D = 2: v = |e|, D = 3: v = |n| / 2
+				const double fc = (double) gco * (double) vi * (double) ciw2 * (ck == 'M' ? -1.0 : -2.0), ft = (double) gco * (double) half;
 				for (int d = 0; d < D; ++d) {
 					gc[d] += fc * (double) tgc[d];
-					gt[d] += ft * ((double) tgt[d] + (double) ui[d] * ((double) tile - (double) angSum));
+					gt[d] += ft * ((double) tgt[d] + (double) ui[d] * (double) tile);
 				}
 			} else if (G) {
 				for (int d = 0; d < D; ++d) { gc[d] += (double) tgc[d]; gt[d] += (double) tgt[d]; }

@@ -160,7 +160,10 @@ __device__ __forceinline__ bool wait_grid(GridBar *bar, unsigned int target)
 // Three lines rotate: line k mod 3 serves the k-th sum; a CTA that has passed sum k knows that all have read line
 // k - 1, which CTA 0 clears then for sum k + 2.
 // ---------------------------------------------------------------------------
-constexpr int kSumMargin = 24;             // a sum may grow by 2^24 from one iteration to the next
+#ifndef SA_SUM_MARGIN
+#define SA_SUM_MARGIN 24                   // tests build with less, so that sums leave their frames often
+#endif
+constexpr int kSumMargin = SA_SUM_MARGIN;  // a sum may grow by 2^24 from one iteration to the next
 constexpr int kSumDigits = 5, kSumDigitBits = 26, kSumWords = 16;
 constexpr int kSumMaxCtas = 255;           // CTA count field: 8 bits
 

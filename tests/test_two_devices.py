@@ -1,19 +1,11 @@
 """One process, two devices: the host code runs over a CUDA runtime without a GPU (fake_cudart.cpp), the same calls first on
 device 0, then on device 1.  Limits that a kernel has per device (dynamic shared memory) are raised on both: no launch is
 refused, and both devices run the same kernels."""
-import os
-import subprocess
-import sys
-
 import pytest
 
-HERE = os.path.dirname(os.path.abspath(__file__))
-ROOT = os.path.dirname(HERE)
-CUDA = "/usr/local/cuda/include"
+import fake_cuda
 
 RUN = """
-import sys
-sys.path.insert(0, {root!r})
 from shape_atrophy_gb300 import _lib, api, problems
 frame = problems.demo_strip(101, 31, timeEnd=0.01)
 layered = problems.annulus_layered(steps=1)
@@ -29,21 +21,7 @@ for device in (0, 1):
 
 @pytest.fixture(scope="module")
 def launches(tmp_path_factory):
-    if not os.path.exists(os.path.join(CUDA, "cuda_runtime_api.h")):
-        pytest.skip("no CUDA headers")
-    from shape_atrophy_gb300 import build
-    build.build()
-    out = tmp_path_factory.mktemp("cudart")
-    with open(out / "versions", "w") as f:
-        f.write("libcudart.so.13 { global: *; };\n")
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", CUDA, "-Wl,-soname,libcudart.so.13",
-                    f"-Wl,--version-script={out}/versions", "-o", str(out / "libcudart.so.13"),
-                    os.path.join(HERE, "fake_cudart.cpp")], check=True)
-    log = out / "log"
-    env = dict(os.environ, LD_LIBRARY_PATH=str(out), FAKE_CUDART_LOG=str(log))
-    r = subprocess.run([sys.executable, "-c", RUN.format(root=ROOT)], env=env, capture_output=True, text=True, timeout=600)
-    lines = [l.split(" ", 1) for l in log.read_text().splitlines()] if log.exists() else []
-    return r, lines
+    return fake_cuda.run(RUN, tmp_path_factory.mktemp("cudart"))
 
 
 def test_calls_succeed_on_both_devices(launches):

@@ -36,6 +36,7 @@ struct sa_context {
 	cudaStream_t side = nullptr;                    // work that overlaps the host's set-up (target varifold rows)
 	cudaEvent_t e0 = nullptr, e1 = nullptr;
 	cudaEvent_t sideIn = nullptr, sideOut = nullptr;
+	bool planned = false, noPlan = false;           // the running call: has a velocity plan, does without one
 	std::string err;
 };
 
@@ -62,13 +63,13 @@ struct Pool {                 // device allocations of one call, freed at the en
 	bool ordered = false;
 	explicit Pool(cudaStream_t st, bool streamOrdered = false) : s(st), ordered(streamOrdered) {}
 	~Pool() { release(); }
-	void release()
+	void release(size_t from = 0)          // the allocations from number `from` on
 	{
-		for (void *p : ptrs) {
-			if (ordered) cudaFreeAsync(p, s);
-			else cudaFree(p);
+		for (size_t k = from; k < ptrs.size(); ++k) {
+			if (ordered) cudaFreeAsync(ptrs[k], s);
+			else cudaFree(ptrs[k]);
 		}
-		ptrs.clear();
+		ptrs.resize(from);
 	}
 	template <typename T> T *alloc(size_t n)
 	{
@@ -659,8 +660,10 @@ static void alloc_work(Work &w, const Mesh &m, const Model &md, bool wantTraj, P
 // the plan of the fixed-point persistent CG for the FP64 velocity solves of a layered call (none when device memory
 // for it is short: the solves then take the FP64 kernels)
 template <int D>
-static void plan_velocity_cg(Work &w, const Mesh &m, const Model &md, const double *x0soa, Pool &P)
+static void plan_velocity_cg(sa_context *ctx, Work &w, const Mesh &m, const Model &md, const double *x0soa, Pool &P)
 {
+	ctx->planned = false;
+	if (ctx->noPlan) return;
 	if (md.frame || md.ldmWgt != 0.0 || md.precision != SA_PREC_FP64) return;
 	if (md.cgKernel != SA_CG_AUTO && md.cgKernel != SA_CG_PERSISTENT) return;
 	auto alloc = [&](size_t bytes) -> void * {
@@ -671,7 +674,12 @@ static void plan_velocity_cg(Work &w, const Mesh &m, const Model &md, const doub
 			return nullptr;
 		}
 	};
-	cgfix_plan(m, x0soa, w.cw.smCount, tuning().persistMaxWarps, w.cw.plan, alloc, P.s);
+	const size_t before = P.ptrs.size();
+	if (!cgfix_plan(m, x0soa, w.cw.smCount, tuning().persistMaxWarps, w.cw.plan, alloc, P.s)) {
+		P.release(before);                   // what the call allocates next finds the memory that it had without a plan
+		w.cw.plan = CgPlan();
+	}
+	ctx->planned = w.cw.plan.ok;
 }
 
 __global__ void k_to_f32(long n, const double *a, float *b)
@@ -966,7 +974,7 @@ static int forward_impl(sa_context *ctx, const sa_element_object *obj, const dou
 	std::vector<double> tv = to_host(tauVarMat, (size_t) tauVarNum * objNum, s);
 	Work w;
 	alloc_work<D>(w, m, md, lmkStk != nullptr, P);
-	plan_velocity_cg<D>(w, m, md, x0, P);
+	plan_velocity_cg<D>(ctx, w, m, md, x0, P);
 	{   // initial element orientation for the Jacobian sign check
 		double *xa = P.alloc<double>((size_t) m.N * D);
 		launch_soa_to_aos(m.N, D, x0, xa, s);
@@ -1089,7 +1097,7 @@ static int gradient_impl(sa_context *ctx, const sa_element_object *obj, const do
 	const double *tvl = P.dev(tgt->elmVolVec, (size_t) tgt->tgtElmNum);
 	Work w;
 	alloc_work<D>(w, m, md, false, P);
-	plan_velocity_cg<D>(w, m, md, x0, P);
+	plan_velocity_cg<D>(ctx, w, m, md, x0, P);
 	{
 		double *xa = P.alloc<double>((size_t) m.N * D);
 		launch_soa_to_aos(m.N, D, x0, xa, s);
@@ -1417,7 +1425,7 @@ static int adjoint_impl(sa_context *ctx, const sa_element_object *obj, const dou
 	const double *tvl = P.dev(tgt->elmVolVec, (size_t) tgt->tgtElmNum);
 	Work w;
 	alloc_work<D>(w, m, md, true, P);
-	plan_velocity_cg<D>(w, m, md, x0, P);
+	plan_velocity_cg<D>(ctx, w, m, md, x0, P);
 	const long n = (long) m.N * D, N = m.N;
 	const int T = md.timeNum;
 	const double dt = md.timeStp;
@@ -1603,7 +1611,7 @@ struct Session : SessionBase {
 			tvl = P.dev(tgt->elmVolVec, (size_t) Vt);
 		}
 		alloc_work<D>(w, m, md, false, P);
-		plan_velocity_cg<D>(w, m, md, x0, P);
+		plan_velocity_cg<D>(ctx, w, m, md, x0, P);
 		double *xa = P.alloc<double>((size_t) m.N * D);
 		launch_soa_to_aos(m.N, D, x0, xa, s);
 		k_init_sign<D><<<grid_for(m.E), kBlock, 0, s>>>(m.E, m.elmVtx, xa, m.sign0);
@@ -1748,6 +1756,22 @@ struct Session : SessionBase {
 		}
 	}
 };
+
+// a call that plans its velocity solves; when device memory runs out after the plan, once more without it
+template <typename F>
+static int planning(sa_context *ctx, F &&f)
+{
+	ctx->planned = ctx->noPlan = false;
+	try {
+		return f();
+	} catch (const CudaError &e) {
+		if (e.e != cudaErrorMemoryAllocation || !ctx->planned) throw;
+		cudaGetLastError();
+	}
+	struct Off { bool &b; ~Off() { b = false; } } off{ctx->noPlan};
+	ctx->noPlan = true;
+	return f();
+}
 
 template <typename F>
 static int guarded(sa_context *ctx, F &&f)
@@ -2486,7 +2510,7 @@ int sa_forward(sa_context *ctx, const sa_element_object *obj, const double *lmkI
                const sa_target *tgt, const double *tauVarMat, int tauVarNum, int objNum, double *lmkStk,
                double *tauMat, double *objVec, sa_solve_info *info)
 {
-	return sa::guarded(ctx, [&]() {
+	return sa::guarded(ctx, [&]() { return sa::planning(ctx, [&]() {
 		SA_REQUIRE(obj && prm && lmkIniMat, "null argument");
 		if (obj->dim == 2)
 			return sa::forward_impl<2>(ctx, obj, lmkIniMat, prm, tgt, tauVarMat, tauVarNum, objNum, lmkStk, tauMat,
@@ -2494,7 +2518,7 @@ int sa_forward(sa_context *ctx, const sa_element_object *obj, const double *lmkI
 		SA_REQUIRE(obj->dim == 3, "dim must be 2 or 3");
 		return sa::forward_impl<3>(ctx, obj, lmkIniMat, prm, tgt, tauVarMat, tauVarNum, objNum, lmkStk, tauMat,
 		                           objVec, info);
-	});
+	}); });
 }
 
 int sa_varifold(sa_context *ctx, const sa_element_object *obj, const double *lmkMat, const sa_target *tgt,
@@ -2517,7 +2541,7 @@ int sa_session_create(sa_context *ctx, const sa_element_object *obj, const doubl
 {
 	if (!out) return SA_ERR_ARG;
 	*out = nullptr;
-	return sa::guarded(ctx, [&]() {
+	return sa::guarded(ctx, [&]() { return sa::planning(ctx, [&]() {
 		SA_REQUIRE(obj && prm && lmkIniMat, "null argument");
 		sa::SessionBase *impl;
 		if (obj->dim == 2) impl = new sa::Session<2>(ctx, obj, lmkIniMat, prm, tgt, tauVarVec, tauVarNum);
@@ -2527,7 +2551,7 @@ int sa_session_create(sa_context *ctx, const sa_element_object *obj, const doubl
 		}
 		*out = new sa_session{impl};
 		return SA_OK;
-	});
+	}); });
 }
 
 int sa_session_step(sa_session *s, int nsteps, int *stepsDone)
@@ -2545,12 +2569,12 @@ int sa_objective_gradient(sa_context *ctx, const sa_element_object *obj, const d
                           double *objOut, double *gradOut, sa_solve_info *info)
 {
 	if (!ctx || !obj || !prm) return SA_ERR_ARG;
-	return sa::guarded(ctx, [&]() {
+	return sa::guarded(ctx, [&]() { return sa::planning(ctx, [&]() {
 		if (obj->dim == 2)
 			return sa::gradient_impl<2>(ctx, obj, lmkIniMat, prm, tgt, tauVarVec, tauVarNum, objOut, gradOut, info);
 		SA_REQUIRE(obj->dim == 3, "dim must be 2 or 3");
 		return sa::gradient_impl<3>(ctx, obj, lmkIniMat, prm, tgt, tauVarVec, tauVarNum, objOut, gradOut, info);
-	});
+	}); });
 }
 
 int sa_objective_adjoint(sa_context *ctx, const sa_element_object *obj, const double *lmkIniMat, const sa_params *prm,
@@ -2558,14 +2582,14 @@ int sa_objective_adjoint(sa_context *ctx, const sa_element_object *obj, const do
                          double *gradBump, double *gradLayer, double *gradTau0, double *gradX0, sa_solve_info *info)
 {
 	if (!obj || !lmkIniMat || !prm || !tgt || !tauVarVec) return SA_ERR_ARG;
-	return sa::guarded(ctx, [&]() {
+	return sa::guarded(ctx, [&]() { return sa::planning(ctx, [&]() {
 		if (obj->dim == 2)
 			return sa::adjoint_impl<2>(ctx, obj, lmkIniMat, prm, tgt, tauVarVec, tauVarNum, objOut, gradBump,
 			                           gradLayer, gradTau0, gradX0, info);
 		SA_REQUIRE(obj->dim == 3, "dim must be 2 or 3");
 		return sa::adjoint_impl<3>(ctx, obj, lmkIniMat, prm, tgt, tauVarVec, tauVarNum, objOut, gradBump, gradLayer,
 		                           gradTau0, gradX0, info);
-	});
+	}); });
 }
 
 int sa_session_stream(sa_session *s, int nsteps, int stride, double *lmkOut, double *tauOut, int maxSnapshots,

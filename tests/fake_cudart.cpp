@@ -1,7 +1,8 @@
 // A CUDA runtime without a GPU, for the CPU tests of the host code: two devices, device memory on the heap, kernels that do
 // nothing.  A launch is refused, as on a GPU, when it asks for more shared memory than its kernel may use on the current
 // device: 48 KB, static and dynamic together, until cudaFuncSetAttribute raises the kernel's limit there.  Every launch is
-// written to the file named by FAKE_CUDART_LOG: device, kernel.
+// written to the file named by FAKE_CUDART_LOG: device, kernel.  FAKE_CUDART_MEMORY: bytes of device memory, read at every
+// allocation.
 #include <cuda_runtime_api.h>
 #include <cstdio>
 #include <cstdlib>
@@ -18,6 +19,7 @@ std::mutex mu;
 std::map<const void *, std::string> names;
 std::map<std::pair<int, const void *>, size_t> limits;
 std::map<char *, size_t> blocks;
+size_t used = 0, most = 0;
 thread_local int device = 0;
 thread_local cudaError_t last = cudaSuccess;
 struct Config { dim3 g, b; size_t smem; cudaStream_t s; };
@@ -45,10 +47,13 @@ cudaError_t launch(const void *f, size_t smem)
 
 cudaError_t alloc(void **p, size_t n)
 {
-	*p = std::calloc(1, n ? n : 1);
-	if (!*p) return ret(cudaErrorMemoryAllocation);
 	std::lock_guard<std::mutex> g(mu);
+	const char *cap = std::getenv("FAKE_CUDART_MEMORY");
+	*p = cap && used + n > (size_t) std::atoll(cap) ? nullptr : std::calloc(1, n ? n : 1);
+	if (!*p) return ret(cudaErrorMemoryAllocation);
 	blocks[(char *) *p] = n;
+	used += n;
+	if (used > most) most = used;
 	return cudaSuccess;
 }
 
@@ -56,6 +61,7 @@ cudaError_t release(void *p)
 {
 	if (!p) return cudaSuccess;
 	std::lock_guard<std::mutex> g(mu);
+	used -= blocks[(char *) p];
 	blocks.erase((char *) p);
 	std::free(p);
 	return cudaSuccess;
@@ -64,6 +70,9 @@ char symbol[1 << 20];
 }  // namespace
 
 extern "C" {
+// most device memory in use at once since the last call
+size_t fake_cudart_most() { const size_t m = most; most = used; return m; }
+
 void **__cudaRegisterFatBinary(void *) { static void *h; return &h; }
 void __cudaRegisterFatBinaryEnd(void **) {}
 void __cudaUnregisterFatBinary(void **) {}

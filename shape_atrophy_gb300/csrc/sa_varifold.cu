@@ -233,7 +233,8 @@ __device__ __forceinline__ double cen_knl_grad(int type, double d2, double iw2, 
 	const double q = d2 * iw2;
 	const unsigned long long r = pair_sqrt((unsigned) __double2hiint(q), (unsigned) __double2loint(q));
 	if (r == kPairFar) {
-		const double s = sqrt_nr(q), ex = exp_tab(-s, tab);
+		// (an infinite distance gives 0, not inf * 0; NaN stays)
+		const double s = sqrt_nr(q > DBL_MAX ? DBL_MAX : q), ex = exp_tab(-s, tab);
 		cg = ex;
 		return fma(s, ex, ex);
 	}
@@ -372,7 +373,8 @@ __global__ void k_vfd_rows(VfdSet R, VfdSet A, double cA, VfdSet Bs, double cB, 
 	const T nLen = (D == 2 ? vi : (T) 2.0 * vi), half = (D == 2 ? (T) 1.0 : (T) 0.5);
 	double acc = 0.0, gc[D], gt[D];
 	for (int d = 0; d < D; ++d) { gc[d] = 0.0; gt[d] = 0.0; }
-	const T ciw = (T) (1.0 / cw), ciw2 = (T) (1.0 / (cw * cw)), diw2 = (T) (1.0 / (dw * dw));
+	// (a width below 2^-512: every pair but a centre with itself is beyond reach, and that one's 0 / w^2 stays 0)
+	const T ciw = (T) (1.0 / cw), ciw2 = (T) (kFixG ? fmin(1.0 / (cw * cw), DBL_MAX) : 1.0 / (cw * cw)), diw2 = (T) (1.0 / (dw * dw));
 	out = out0 + (long) cy * R.n;
 	if (G) { dc = dc0 + (long) cy * D * R.n; dt = dt0 + (long) cy * D * R.n; }
 	for (int set = 0; set < 2; ++set) {

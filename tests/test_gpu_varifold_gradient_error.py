@@ -2,7 +2,8 @@
 
 1. Nodes on a grid of 2^-20: centres and their differences are exact in FP64 wherever the shape lies, so the gradient of a
    curve moved by whole numbers keeps its bits.
-2. Against sums in numpy's long double (64 bits and more), relative in the 2-norm, root mean square over eight shapes: at
+2. A width whose square leaves the range of FP64 gives what a width far below every distance gives.
+3. Against sums in numpy's long double (64 bits and more), relative in the 2-norm, root mean square over eight shapes: at
    most 1.5 times the error of the same pair terms in numpy's FP64.  Two FP64 evaluations that differ in the order of their
    sums differ by less than that over so many shapes; the bound leaves no room for a term that cancels (2 to 2.8 times)."""
 import numpy as np
@@ -124,3 +125,28 @@ def test_error_against_extended_precision(cen, direction, width):
     here, plain = (float(np.sqrt(np.mean(np.square(e)))) for e in (here, plain))
     print(f"{cen} x {direction} {width}: {here:.2e}, FP64 in numpy {plain:.2e}")
     assert here <= 1.5 * plain
+
+
+@pytest.mark.parametrize("cen", ["G", "M"])
+@pytest.mark.parametrize("k", [0, 1])
+def test_width_below_every_distance(cen, k):
+    """Only an element's pair with itself counts, whatever the width."""
+    from shape_atrophy_gb300 import api, mesh
+    obj, lmk = _shape(k, np.random.default_rng(3))
+    spec = dict(dim=lmk.shape[0], elmObj=obj, lmkIniMat=lmk,
+                tgt=mesh.varifold_target(lmk + 0.02 * np.sin(3 * lmk[::-1]), obj["vfdVtxMat"]))
+    out = [api.varifold(dict(spec, vfd=(cen, w, "B", 1.0)), lmk, grad=True) for w in (1e-5, 1e-200)]
+    assert np.abs(out[0][1]).max() > 0.0
+    assert out[0][0] == out[1][0]
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("cen", ["G", "C", "M"])
+def test_a_target_centre_that_is_not_a_number(cen):
+    from shape_atrophy_gb300 import api, mesh
+    obj, lmk = _shape(0, np.random.default_rng(3))
+    tgt = [np.array(t, copy=True) for t in mesh.varifold_target(lmk + 0.01, obj["vfdVtxMat"])]
+    tgt[0][0, 3] = np.nan
+    spec = dict(dim=2, elmObj=obj, lmkIniMat=lmk, tgt=tuple(tgt), vfd=(cen, 0.1, "B", 1.0))
+    value, grad = api.varifold(spec, lmk, grad=True)
+    assert np.isnan(value) and np.isnan(grad).any() and np.isnan(api.varifold(spec, lmk))

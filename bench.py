@@ -530,19 +530,22 @@ def main():
     value = ws * K / (ms_max / 1000.0)
     hbm, peak_kind = peaks()
     persistent = 0 < 4 * k_cnt < cg_iters              # one launch per solve, not one per iteration
-    kname = (("k_cg_fix" if args.precision == "fp64" else "k_cg_persist") +
-             " (whole velocity CG solve: matvec, vector updates, dots)" if persistent
-             else "k_cg_spmv (velocity block matvec + dot)")
-    avg_launch_s = (k_ms / k_cnt) / 1000.0 if k_cnt else float("nan")
     N_, E_ = spec["lmkIniMat"].shape[1], spec["elmObj"]["elmVtxMat"].shape[1]
     D_ = int(spec["dim"])
+    # the kernel that ran: the fixed-point solver reports the FP64 flops of its vector work alone, 2 (7 + D) per entry and
+    # iteration; above 19 32-row slices per SM it is the form with several chunks per CTA
+    kernel = "k_cg_persist" if persistent else "k_cg_spmv"
+    if persistent and args.precision == "fp64" and abs(k_flops / cg_iters - 2.0 * (7 + D_) * N_ * D_) < 1.0:
+        kernel = "k_cg_fix" if N_ <= 32 * 19 * api.device_name(local)[1] else "k_cg_fix_many"
+    kname = kernel + (" (whole velocity CG solve: matvec, vector updates, dots)" if persistent else
+                      " (velocity block matvec + dot)")
+    avg_launch_s = (k_ms / k_cnt) / 1000.0 if k_cnt else float("nan")
     alg = algorithmic_bytes(N_, E_, D_, 4 if args.precision == "mixed" else 8)
     iters_per_launch = cg_iters / k_cnt if (k_cnt and persistent) else 1.0
     bytes_per_launch = alg["iteration"] * iters_per_launch if persistent else alg["matvec"]
     achieved = bytes_per_launch / avg_launch_s / 1e9 if k_cnt else None
     traffic = None
-    tfile = os.path.join(ROOT, "profiles", (("k_cg_fix" if args.precision == "fp64" else "k_cg_persist") if persistent
-                                              else "k_cg_spmv") + f"_shell_l5_{args.precision}_traffic.txt")
+    tfile = os.path.join(ROOT, "profiles", f"{kernel}_shell_l5_{args.precision}_traffic.txt")
     if os.path.exists(tfile) and args.workload == "shell":
         for line in open(tfile):
             if line.startswith("dram_bytes_per_iteration:") and cg_iters:
@@ -583,7 +586,7 @@ def main():
                            "SM clock sampled during the timed steps",
             "flops_model": ("2 x 10 x vector entries per CG iteration (per entry the x, r, p, s updates, three dot terms "
                             "and a row of the 3x3 block-Jacobi inverse); the operator's products are summed on the "
-                            "integer pipes" if fp64 and persistent else
+                            "integer pipes" if kernel.startswith("k_cg_fix") else
                             "2 x (9 x operator slots + 10 x vector entries) per CG iteration (assembled 3x3 blocks; "
                             "per entry the x, r, p, s updates, three dot terms and a row of the 3x3 block-Jacobi "
                             "inverse)")}

@@ -49,7 +49,9 @@ extern "C" {
 #define SA_ELA_FRAME          0   /* reference frame elasticity, K-preconditioned CG */
 #define SA_ELA_ISOTROPIC      1   /* layered isotropic elasticity, block-Jacobi PCG */
 
-#define SA_PREC_FP64          0   /* FP64, or fixed point of at least its precision (solver products, pair terms) */
+#define SA_PREC_FP64          0   /* FP64; solver products and varifold pair terms in fixed point: 55 bits and more
+                                     of the largest entry of a row, a vector's part or a tile, as accurate as FP64
+                                     in norm, smaller entries with fewer bits of their own */
 #define SA_PREC_MIXED         1   /* FP32 operators, FP64 dots/residuals + refinement */
 
 #define SA_CG_AUTO            0   /* persistent CG kernel: FP64 block systems with fixed-point products when their plan
@@ -218,7 +220,8 @@ int sa_objective_adjoint(sa_context *ctx, const sa_element_object *obj, const do
  * objective: an optimiser's line search that calls it hundreds of times on
  * a GPU whose memory is managed by someone else (MATLAB's gpuArray pool, a
  * serving process with a fixed budget), where cudaMalloc can fail and
- * cudaFree synchronises the whole device.  Same value as sa_varifold.
+ * cudaFree synchronises the whole device.  The value of sa_varifold to
+ * rounding (FP64 pair terms here, fixed point there).
  *   - All inputs must already be memory of the current device (nodes:
  *     N x dim column-major; vfdVtxMat: Vd x dim int32; target Vt x dim,
  *     Vt); host pointers and other GPUs' memory are rejected with

@@ -1329,8 +1329,8 @@ static CgScal run_cg(const Mesh &m, const TM *blk, const TV *dinv, const double 
 		                                   : (const TV *) (const void *) prof->binv64;
 		if (!binv) throw CudaError{cudaErrorInvalidValue, "block-Jacobi CG without block inverses"};
 	}
-	// FP64 velocity solves: the persistent CG with fixed-point matrix products, where its plan exists (at most one
-	// slice per row warp and a halo that fits shared memory)
+	// FP64 velocity solves: the persistent CG with fixed-point matrix products, where its plan exists (one chunk of rows
+	// per CTA, or several; halos that fit shared memory, rows that fit a digit sum)
 	if constexpr (B > 1 && sizeof(TM) == sizeof(double) && sizeof(TX) == sizeof(double)) {
 		if (prof->plan.ok && prof->bar && (prof->cgKernel == SA_CG_AUTO || prof->cgKernel == SA_CG_PERSISTENT)) {
 			k_cg_init_blk<B, TV><<<vec_grid(N, prof->smCount), kCgBlock, 0, s>>>(N, b, q, binv, r, u, part, sc);

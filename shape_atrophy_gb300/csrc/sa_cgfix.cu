@@ -16,8 +16,11 @@
 //     its own) are read into shared memory as two 28-bit digits relative to the halo's largest entry, so a
 //     slot's gather is six shared-memory words instead of two L2 requests;
 //   * the two grid sums of an iteration carry their own barrier (sum_exchange in sa_grid.cuh).
-// The shell's iteration takes 21 us here (43 thousand clocks: products 20, vector updates 6, halo 6, the two grid sums 7),
-// a call 265 -> 192 ms; the 4 096-node annulus, bound by the sums, 8.9 -> 6.2 us; from 97 000 nodes k_cg_fix_many.
+// The shell's iteration takes 21 us here (43 thousand clocks: products 20, vector updates 6, halo 6, the two grid sums 7)
+// instead of 35; the 4 096-node annulus, bound by the sums, 8.9 -> 6.3 us; above 92 416 rows (19 slices on each of 152 SMs)
+// k_cg_fix_many.  What bounds it is latency: of the shell's solve the warps issue in 36 % of the cycles, the integer pipe is
+// busy in 28 %, the multiply pipe in 17 %, the FP64 pipe in 21 %; a waiting warp waits at barriers (grid sums and between
+// phases), then on dependent instructions and on shared and global loads (profiles/k_cg_fix.md).
 // The recurrences, the reducer warp and the stopping rule are those of k_cg_persist (sa_cg.cu): Chronopoulos-Gear
 // in FP64, exact grid sums, bounded waits.
 #include "sa_internal.cuh"
@@ -42,7 +45,7 @@ __host__ __device__ __forceinline__ int row_pack(int e, int s) { return (int) ((
 __host__ __device__ __forceinline__ int row_frame(int w) { return w >> 16; }
 __host__ __device__ __forceinline__ int row_scale(int w) { return (short) w; }
 
-template <int B> constexpr int limb_stride() { return 6; }    // words per halo node: three 8-byte bank pairs, odd, so consecutive nodes spread
+constexpr int kLimbStride = 6;             // words per halo node: three 8-byte bank pairs, odd, so consecutive nodes spread
 template <int B> constexpr int fix_u_stride() { return B == 3 ? 4 : 2; }   // doubles per node of the gather copy
 
 // ---------------------------------------------------------------------------
@@ -343,7 +346,7 @@ struct FixArgs {
 template <int B> size_t fix_smem(int pw, int parts, int haloMax, int colMax, int stages)
 {
 	return (size_t) pw * stages * (256 * B * B + 8) + sizeof(double) * (size_t) pw * 32 * (B * B + B + (parts - 1) * 3 * B) +
-	       sizeof(int) * (size_t) haloMax * (limb_stride<B>() + 1) + sizeof(unsigned short) * (size_t) colMax + 16;
+	       sizeof(int) * (size_t) haloMax * (kLimbStride + 1) + sizeof(unsigned short) * (size_t) colMax + 16;
 }
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned) __cvta_generic_to_shared(p); }
@@ -490,7 +493,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 	extern __shared__ __align__(128) char sdyn[];
 	CgScal *sc = a.sc;
 	if (sc->done) return;                        // set by k_cg_init: the same for every CTA
-	constexpr int S = limb_stride<B>(), U = fix_u_stride<B>(), BB = B * B;
+	constexpr int S = kLimbStride, U = fix_u_stride<B>(), BB = B * B;
 	constexpr unsigned kSlot = 256 * BB;         // bytes of one slot of a slice
 	const int nctas = gridDim.x, lc = blockIdx.x, pw = a.pw;
 	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, W = blockDim.x >> 5;
@@ -820,7 +823,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix(const FixArgs a
 }
 
 // ---------------------------------------------------------------------------
-// The same solve for operators of more than one chunk per CTA (97 000 nodes and up).  The CTA takes its per chunks in
+// The same solve for operators of more than one chunk per CTA (more than 92 416 rows).  The CTA takes its per chunks in
 // turn: the row warps multiply one while the staging warps gather and convert the next one's halo.  The warp's operator
 // ring, whose slots carry their columns, runs on from chunk to chunk; the last slots of the first chunk's slices stay in
 // tensor memory.  x, p, s and r of the rows and their block inverses are in global memory, 32 rows of a component together
@@ -850,7 +853,7 @@ template <int B> __host__ __device__ constexpr int many_slot() { return 256 * B 
 // slots in tensor memory
 template <int B> size_t fix_many_smem(int pw, int haloMax, int stages)
 {
-	return (size_t) pw * stages * (many_slot<B>() + 8) + sizeof(int) * (size_t) haloMax * (2 * limb_stride<B>() + 1) +
+	return (size_t) pw * stages * (many_slot<B>() + 8) + sizeof(int) * (size_t) haloMax * (2 * kLimbStride + 1) +
 	       (size_t) pw * tmem_slots<B>(pw) * 64 + 16;
 }
 
@@ -865,7 +868,7 @@ __global__ void __launch_bounds__(32 * kFixMaxWarps, 1) k_cg_fix_many(const FixA
 	extern __shared__ __align__(128) char sdyn[];
 	CgScal *sc = a.sc;
 	if (sc->done) return;
-	constexpr int S = limb_stride<B>(), U = fix_u_stride<B>(), BB = B * B;
+	constexpr int S = kLimbStride, U = fix_u_stride<B>(), BB = B * B;
 	constexpr int kSlot = 256 * BB, kRing = many_slot<B>();
 	const int nctas = gridDim.x, lc = blockIdx.x, pw = a.pw;
 	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, W = blockDim.x >> 5;

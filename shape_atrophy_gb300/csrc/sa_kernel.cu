@@ -424,11 +424,15 @@ __global__ void k_kp_zero(long n, double *x, double *w, const KScal *sc)
 // ---------------------------------------------------------------------------
 // Fixed-point products with the RKHS matrix.  The product with D right-hand sides is N^2 D multiply-adds per
 // iteration, which the FP64 pipe issues at 1.6 per clock per SM: 37 us of a 69 us iteration on the 3131-node strip, where
-// the matrix itself (78 MB) streams from L2 in 5 us.  With the digits below the product takes 20 us there (integer
-// multiply-adds) and the iteration 37 us.  The entries are therefore kept as two 28-bit digits (the bytes
-// of the double; frame: the largest entry, 1 + eps) and multiplied on the integer pipes (sa_limb.cuh); r is converted
-// once per CTA and product into shared memory.  Sums are exact and rounded once, so they do not depend on how rows and
-// columns are dealt out, and the matrix-free form, which converts the same entries on the fly, gives the same bits.
+// the matrix itself (78 MB) streams from L2 in 5 us.  With the digits below the product takes 20 us there and the
+// iteration 37 us.  The entries are therefore kept as two 28-bit digits (the bytes of the double; one frame for all of
+// them, the largest entry's, |1 + eps| or 1) and multiplied on the integer pipes (sa_limb.cuh); r is converted once per CTA
+// and product into shared memory.  Sums are exact but for 7 bits cut at each flush (2^-96 of the largest product over a row) and rounded once, and the matrix-free form, which converts the same entries on the fly and flushes at
+// the same places, gives the same bits.  A far entry is rounded at 2^-55 of the largest, not of itself: in norm the product
+// is as good as FP64's, and so are the solves (shells with orders -1 to 4, widths 0.1 to 1 and ldm 1e-3 to 1 against solves
+// refined in 113 bits: errors 1.00 times those of FP64 products in the geometric mean).
+// What bounds the solve on the strip is latency: issue 33 % of the cycles, integer pipe 30 %, multiply pipe 17 %
+// (profiles/k_kpcg_persist_frame_demo_strip.md).
 // ---------------------------------------------------------------------------
 constexpr int kKpWarps = 16;
 constexpr int kKpRows = 8;          // rows of a block: a warp multiplies 8 rows by 4 columns at a time

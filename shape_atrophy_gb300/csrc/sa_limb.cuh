@@ -15,7 +15,8 @@
 //   sum va vu = 2^56 S2 + 2^28 S1 + S0, S2 = sum a1 u1, S1 = sum (a1 u0 + a0 u1), S0 = sum a0 u0, nothing dropped.  S1 is
 //     formed as M - S2 - S0 from M = sum (a1 + a0)(u1 + u0) (Karatsuba's product), so a product takes three integer
 //     multiply-adds, each about four clocks of a sub-partition, and two 32-bit additions.
-// Each sum stays below 2^63 for up to kLimbMaxTerms products.  A frame of 2047 (an Inf or NaN in the row or the set) gives
+// Each sum stays below 2^63 for up to kLimbMaxTerms products.  So a product with a vector is as good as FP64's in norm, not
+// entry by entry: where a row's terms are 2^-k of its largest entry times the set's largest, it has k bits less.  A frame of 2047 (an Inf or NaN in the row or the set) gives
 // NaN.  An entry above its frame has no digits (0 comes out): the caller's frame covers every entry, or the caller looks
 // for such entries and gives NaN.
 #pragma once
